@@ -149,27 +149,63 @@ __device__ double warp_dot(const double *x, const double *y, int n) {
 // Cyclic Jacobi on the symmetric n x n matrix S (row-major, ld DAV_MAXD,
 // zero outside n x n) by the whole block; eigenvectors accumulate in the
 // columns of V.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an
-// element below 1e-17 sqrt(|a_pp a_qq|) is negligible and set to zero; a
+// element with a_pq^2 <= 1e-34 |a_pp a_qq| is negligible and set to zero; a
 // sweep without rotations ends the iteration.  The n(n-1)/2 rotations of a
 // sweep run as n-1 rounds of n/2 disjoint rotations (round-robin pairing,
 // n padded to even), each round one parallel update of S and V.  The
 // iteration ends at the first round whose matrix has no element above the
 // threshold: the rounds left of that sweep and the sweep without rotations
 // would change no diagonal element and no column of V.  The
-// rotation of a pair is
-//   t = sgn(d b) |b| / (|d| + hypot(d, b)),  d = a_qq - a_pp, b = 2 a_pq,
-//   c = 1 / sqrt(1 + t^2),  s = t c
-// (the smaller root of t^2 + 2 tau t - 1 = 0, tau = d / b, written with one
-// division), evaluated next to the threshold test.
+// rotation of a pair is the smaller root t of t^2 + 2 tau t - 1 = 0, tau =
+// d / b, d = a_qq - a_pp, b = 2 a_pq, by its half angle:
+//   h = 1 / sqrt(d^2 + b^2),  u = (1 + |d| h) / 2,  r = 1 / sqrt(u),
+//   c = u r,  s = sgn(d b) |b| h r / 2,
+// two reciprocal roots after one another and no division; a pair whose
+// d^2 + b^2 leaves the normal range is scaled first.
+//
+// Latency bounds it: about 80 rounds at n = 20, each a chain of the rotation
+// parameters, two block barriers and one 2 x 2 update.  So each thread's
+// elements of the test, the update and V are worked out once, before the
+// rounds, and the test squares instead of taking roots.
 __device__ void block_jacobi(double *S, double *V, int n) {
     __shared__ double cs[DAV_MAXD], sn[DAV_MAXD];
-    __shared__ int pp[DAV_MAXD / 2], qq[DAV_MAXD / 2];
     const int tid = threadIdx.x;
     const int m = (n + 1) & ~1, half = m / 2;
     for (int e = tid; e < DAV_MAXD * DAV_MAXD; e += DT) {
         int i = e / DAV_MAXD, j = e % DAV_MAXD;
         V[e] = (i == j && i < m) ? 1.0 : 0.0;
     }
+    // this thread's elements p < q of the threshold test (warps 1..: at most
+    // two of the 496), numbered by columns
+    int tp[2] = {-1, -1}, tq[2] = {0, 0};
+    if (tid >= 32)
+#pragma unroll
+        for (int w = 0; w < 2; w++) {
+            const int e = tid - 32 + w * (DT - 32);
+            if (e < n * (n - 1) / 2) {
+                int q = 1;
+                while ((q + 1) * q / 2 <= e) q++;
+                tp[w] = e - q * (q - 1) / 2;
+                tq[w] = q;
+            }
+        }
+    // its 2 x 2 block (pair k rows, pair l columns) of S (first half of the
+    // threads), or its two (row, pair) items of V (second half)
+    const bool on_s = tid < DT / 2;
+    const int e0 = on_s ? tid : tid - DT / 2;
+    const int k0 = e0 / half, l0 = e0 - k0 * half;
+    const int e1 = e0 + DT / 2, k1 = e1 / half, l1 = e1 - k1 * half;
+    const bool live0 = on_s ? k0 < half : k0 < m, live1 = !on_s && k1 < m;
+    // the pair of index k in round r: (r, m-1) for k = 0, else r + k and r - k
+    // modulo m-1; smaller one first
+    auto pair_of = [&](int k, int r, int *p, int *q) {
+        int a = r + k, b = r - k;
+        if (a >= m - 1) a -= m - 1;
+        if (b < 0) b += m - 1;
+        if (k == 0) b = m - 1;
+        *p = min(a, b);
+        *q = max(a, b);
+    };
     __syncthreads();
     bool done = m <= 1;
     for (int sweep = 0; sweep < 50 && !done; sweep++) {
@@ -177,37 +213,32 @@ __device__ void block_jacobi(double *S, double *V, int n) {
             // does any element of the matrix still call for a rotation?
             // (asked by warps 1.., beside warp 0's rotation parameters)
             bool above = false;
-            for (int e = tid - 32; e >= 0 && e < n * n; e += DT - 32) {
-                const int p = e / n, q = e - p * n;
-                if (p < q) {
-                    const double apq = S[p * DAV_MAXD + q];
-                    above |= !(fabs(apq) <= 1.0e-17 * sqrt(fabs(S[p * DAV_MAXD + p]) * fabs(S[q * DAV_MAXD + q])) ||
+#pragma unroll
+            for (int w = 0; w < 2; w++)
+                if (tp[w] >= 0) {
+                    const double apq = S[tp[w] * DAV_MAXD + tq[w]];
+                    above |= !(apq * apq <= 1.0e-34 * fabs(S[tp[w] * (DAV_MAXD + 1)] * S[tq[w] * (DAV_MAXD + 1)]) ||
                                apq == 0.0);
                 }
-            }
-            if (tid < half) {  // pair k of round r: (m-1, r) and (r+k, r-k) mod m-1
-                int a, b;
-                if (tid == 0) {
-                    a = r;
-                    b = m - 1;
-                } else {
-                    a = (r + tid) % (m - 1);
-                    b = (r - tid + (m - 1)) % (m - 1);
-                }
-                int p = min(a, b), q = max(a, b);
-                double apq = S[p * DAV_MAXD + q];
-                double app = S[p * DAV_MAXD + p], aqq = S[q * DAV_MAXD + q];
-                const double d = aqq - app, b2 = 2.0 * apq;
-                double t = fabs(b2) / (fabs(d) + hypot(d, b2));
-                if (d != 0.0 && ((d > 0.0) != (b2 > 0.0))) t = -t;
-                const double ct = rsqrt(1.0 + t * t);
+            if (tid < half) {
+                int p, q;
+                pair_of(tid, r, &p, &q);
+                const double apq = S[p * DAV_MAXD + q];
+                const double app = S[p * DAV_MAXD + p], aqq = S[q * DAV_MAXD + q];
                 double c = 1.0, s = 0.0;
-                if (!(fabs(apq) <= 1.0e-17 * sqrt(fabs(app) * fabs(aqq)) || apq == 0.0)) {
-                    c = ct;
-                    s = t * ct;
+                if (!(apq * apq <= 1.0e-34 * fabs(app * aqq) || apq == 0.0)) {
+                    double d = aqq - app, b = 2.0 * apq, h2 = fma(d, d, b * b);
+                    if (!(h2 > 1.0e-290 && h2 < 1.0e290)) {
+                        const double f = 1.0 / fmax(fabs(d), fabs(b));
+                        d *= f;
+                        b *= f;
+                        h2 = fma(d, d, b * b);
+                    }
+                    const double h = rsqrt(h2), u = fma(0.5 * fabs(d), h, 0.5), ru = rsqrt(u);
+                    c = u * ru;
+                    s = 0.5 * fabs(b) * h * ru;
+                    if (d != 0.0 && ((d > 0.0) != (b > 0.0))) s = -s;
                 }
-                pp[tid] = p;
-                qq[tid] = q;
                 cs[tid] = c;
                 sn[tid] = s;
             }
@@ -215,31 +246,38 @@ __device__ void block_jacobi(double *S, double *V, int n) {
                 done = true;
                 break;
             }
-            // S <- J^T S J on the 2x2 blocks of (pair k rows, pair l columns)
-            // by the first half of the block, V <- V J by the second
-            for (int idx = tid; tid < DT / 2 && idx < half * half; idx += DT / 2) {
-                const int k = idx / half, l = idx % half;
-                const int pk = pp[k], qk = qq[k], pl = pp[l], ql = qq[l];
-                const double ck = cs[k], sk = sn[k], cl = cs[l], sl = sn[l];
-                double b00 = S[pk * DAV_MAXD + pl], b01 = S[pk * DAV_MAXD + ql];
-                double b10 = S[qk * DAV_MAXD + pl], b11 = S[qk * DAV_MAXD + ql];
-                double t00 = cl * b00 - sl * b01, t01 = sl * b00 + cl * b01;
-                double t10 = cl * b10 - sl * b11, t11 = sl * b10 + cl * b11;
-                double n00 = ck * t00 - sk * t10, n01 = ck * t01 - sk * t11;
-                double n10 = sk * t00 + ck * t10, n11 = sk * t01 + ck * t11;
-                if (k == l) n01 = n10 = 0.0;  // annihilated (or negligible) element
-                S[pk * DAV_MAXD + pl] = n00;
-                S[pk * DAV_MAXD + ql] = n01;
-                S[qk * DAV_MAXD + pl] = n10;
-                S[qk * DAV_MAXD + ql] = n11;
-            }
-            for (int idx = tid - DT / 2; idx >= 0 && idx < m * half; idx += DT / 2) {
-                const int i = idx / half, l = idx % half;
-                const int pl = pp[l], ql = qq[l];
-                const double cl = cs[l], sl = sn[l];
-                double vp = V[i * DAV_MAXD + pl], vq = V[i * DAV_MAXD + ql];
-                V[i * DAV_MAXD + pl] = cl * vp - sl * vq;
-                V[i * DAV_MAXD + ql] = sl * vp + cl * vq;
+            // S <- J^T S J on the 2x2 blocks, V <- V J
+            if (on_s) {
+                if (live0) {
+                    int pk, qk, pl, ql;
+                    pair_of(k0, r, &pk, &qk);
+                    pair_of(l0, r, &pl, &ql);
+                    const double ck = cs[k0], sk = sn[k0], cl = cs[l0], sl = sn[l0];
+                    const double b00 = S[pk * DAV_MAXD + pl], b01 = S[pk * DAV_MAXD + ql];
+                    const double b10 = S[qk * DAV_MAXD + pl], b11 = S[qk * DAV_MAXD + ql];
+                    const double t00 = cl * b00 - sl * b01, t01 = sl * b00 + cl * b01;
+                    const double t10 = cl * b10 - sl * b11, t11 = sl * b10 + cl * b11;
+                    const bool dia = k0 == l0;  // annihilated (or negligible) element
+                    S[pk * DAV_MAXD + pl] = ck * t00 - sk * t10;
+                    S[pk * DAV_MAXD + ql] = dia ? 0.0 : ck * t01 - sk * t11;
+                    S[qk * DAV_MAXD + pl] = dia ? 0.0 : sk * t00 + ck * t10;
+                    S[qk * DAV_MAXD + ql] = sk * t01 + ck * t11;
+                }
+            } else {
+                if (live0) {
+                    int p, q;
+                    pair_of(l0, r, &p, &q);
+                    const double c = cs[l0], s = sn[l0], vp = V[k0 * DAV_MAXD + p], vq = V[k0 * DAV_MAXD + q];
+                    V[k0 * DAV_MAXD + p] = c * vp - s * vq;
+                    V[k0 * DAV_MAXD + q] = s * vp + c * vq;
+                }
+                if (live1) {
+                    int p, q;
+                    pair_of(l1, r, &p, &q);
+                    const double c = cs[l1], s = sn[l1], vp = V[k1 * DAV_MAXD + p], vq = V[k1 * DAV_MAXD + q];
+                    V[k1 * DAV_MAXD + p] = c * vp - s * vq;
+                    V[k1 * DAV_MAXD + q] = s * vp + c * vq;
+                }
             }
             __syncthreads();
         }
@@ -747,38 +785,57 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b) {
         s.vecR[i + k * D] = (i < dimIter) ? V[i * DAV_MAXD + k] : 0.0;
     }
     __syncthreads();
-    if (tid == 0) {
-        // sort (mod_davidson.f90:620-640)
-        for (int i = 0; i < dimIter; i++) lw[i] = i + 1;
-        for (int i = 0; i < dimIter - 1; i++)
-            for (int j = i + 1; j < dimIter; j++)
-                if (vR[lw[j] - 1] < vR[lw[i] - 1]) {
-                    int t = lw[j];
-                    lw[j] = lw[i];
-                    lw[i] = t;
-                }
+    // sort (mod_davidson.f90:620-640): position = number of smaller values;
+    // equal values keep the order that the reference's exchanges leave
+    if (tid < 32) {
+        int rank = 0;
+        bool tie = false;
+        if (tid < dimIter) {
+            const double x = vR[tid];
+            for (int j = 0; j < dimIter; j++) {
+                rank += vR[j] < x;
+                tie |= j != tid && !(vR[j] < x) && !(x < vR[j]);
+            }
+        }
+        tie = __any_sync(0xffffffffu, tie);
+        if (tid < dimIter) lw[tie ? tid : rank] = tid + 1;
+        __syncwarp();
+        if (tie && tid == 0)
+            for (int i = 0; i < dimIter - 1; i++)
+                for (int j = i + 1; j < dimIter; j++)
+                    if (vR[lw[j] - 1] < vR[lw[i] - 1]) {
+                        int t = lw[j];
+                        lw[j] = lw[i];
+                        lw[i] = t;
+                    }
+        __syncwarp();
         // root tracking by largest component (mod_davidson.f90:227-251),
         // searched over the positions not yet given to a root: the
         // reference also searches the assigned ones and, when one of them
         // wins, gives one eigenvector to two roots, whose collapse then
         // orthonormalises a repeated vector (division by zero); wherever the
-        // reference assigns distinct vectors the choice is the same
-        if (!s.lowest) {
-            for (int iroot = 1; iroot <= nroot; iroot++) {
-                double t1 = 0.0;
-                int i = iroot;
-                for (int j = iroot; j <= dimIter; j++) {
-                    double t2 = fabs(V[(iroot - 1) * DAV_MAXD + (lw[j - 1] - 1)]);
-                    if (t2 > t1) {
-                        t1 = t2;
-                        i = j;
+        // reference assigns distinct vectors the choice is the same.  Lane j
+        // holds position j; the first position of the largest component wins
+        if (!s.lowest)
+            for (int iroot = 0; iroot < nroot; iroot++) {
+                const int mine = tid < dimIter ? lw[tid] : 0;
+                double best = tid >= iroot && tid < dimIter ? fabs(V[iroot * DAV_MAXD + (mine - 1)]) : 0.0;
+                int at = best > 0.0 ? tid : iroot;
+                if (!(best > 0.0)) best = 0.0;
+                for (int o = 16; o > 0; o >>= 1) {
+                    const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+                    const int oa = __shfl_xor_sync(0xffffffffu, at, o);
+                    if (ob > best || (ob == best && oa < at)) {
+                        best = ob;
+                        at = oa;
                     }
                 }
-                int idx = lw[i - 1];
-                for (int j = 1; j <= i - iroot; j++) lw[i - j] = lw[i - j - 1];
-                lw[iroot - 1] = idx;
+                const int idx = __shfl_sync(0xffffffffu, mine, at);
+                const int left = __shfl_up_sync(0xffffffffu, mine, 1);
+                if (tid > iroot && tid <= at) lw[tid] = left;
+                if (tid == iroot) lw[tid] = idx;
+                __syncwarp();
             }
-        }
     }
     __syncthreads();
     if (tid < dimIter) {
