@@ -318,11 +318,11 @@ int davidson(const cpsd_params *p, i64 n, i64 nroot, double *fileEV, const doubl
     StepThrottle &th = throttle();
     CPSD_TRY(th.init());
     for (i64 it = 1; it <= p->davidson_cyc + 2; it++) {
-        CPSD_TRY(dav_step_launch(st, b));
+        CPSD_TRY(dav_step_launch(st, b, n, (int)nroot, (int)D));
         CPSD_TRY(th.mark(it));
         if (((volatile int *)mb)[0] == 0) break;
         CPSD_TRY(sigma(b.W, n, b.AW, n, nroot));
-        CPSD_TRY(dav_abar_launch(st, b));
+        CPSD_TRY(dav_abar_launch(st, b, (int)nroot, (int)D));
         CPSD_TRY(th.wait(it));
     }
     int *hdr = (int *)mailbox();

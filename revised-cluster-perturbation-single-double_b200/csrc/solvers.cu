@@ -1,35 +1,101 @@
 // Device-resident Davidson (src/lib_cc/mod_davidson.f90:40-728) and DIIS
-// (src/libsrint/dosodiis2_d.f:1-119, dodiis.f, minv.f) for the small CIS /
-// R1 spaces: one CTA owns the whole subspace logic, so an iteration costs
-// one step launch + the batched sigma contraction + one Ritz-matrix update.
+// (src/libsrint/dosodiis2_d.f:1-119, dodiis.f, minv.f): one cluster of CTAs
+// owns the whole subspace logic, so an iteration costs one step launch + the
+// batched sigma contraction + one Ritz-matrix update.
 #include "solvers.cuh"
+
+#include <algorithm>
+#include <atomic>
+
+#include <cooperative_groups.h>
 
 namespace cpsd {
 
 namespace {
-constexpr int DT = 512;  // threads of the single-CTA solver kernels
+namespace cg = cooperative_groups;
 
-__device__ double block_sum(double v, double *sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    __syncthreads();
-    if (l == 0) sh[w] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double r = 0.0;
-        for (int i = 0; i < DT / 32; i++) r += sh[i];
-        sh[DT / 32] = r;
+constexpr int DT = 512;  // threads of a solver CTA
+
+// The CTAs that own one subspace: a thread-block cluster (one CTA for short
+// vectors), CTA r holding elements [lo, hi) of every vector.  Sums over whole
+// vectors are formed per CTA and exchanged through distributed shared memory:
+// every CTA then adds the partial sums in rank order, so all of them see the
+// same bits and follow the same control flow without a broadcast.
+struct Team {
+    int size, rank, lo, hi;
+    int flip = 0;
+    __device__ Team(int n) {  // the cluster's own split of n elements
+        const cg::cluster_group c = cg::this_cluster();
+        size = (int)c.num_blocks();
+        rank = (int)c.block_rank();
+        const int chunk = ((n + size - 1) / size + 31) & ~31;
+        lo = min(n, rank * chunk);
+        hi = min(n, lo + chunk);
     }
-    __syncthreads();
-    double r = sh[DT / 32];
-    __syncthreads();
-    return r;
+    __device__ void sync() const {
+        if (size > 1) cg::this_cluster().sync();
+        else __syncthreads();
+    }
+    // the buffer of the next exchange (of two: a CTA that fills it has passed
+    // the exchange after its last use, so nobody reads it any more)
+    __device__ double *next(double *buf, int stride) {
+        flip ^= 1;
+        return buf + flip * stride;
+    }
+    // sum (or maximum) over the CTAs of entry e of an exchange buffer, to be
+    // called after sync()
+    __device__ double sum(const double *part, int e) const {
+        if (size == 1) return part[e];
+        double t = 0.0;
+        for (int r = 0; r < size; r++) t += cg::this_cluster().map_shared_rank(const_cast<double *>(part), r)[e];
+        return t;
+    }
+    __device__ double amax(const double *part, int e) const {
+        if (size == 1) return part[e];
+        double t = -1.0;
+        for (int r = 0; r < size; r++)
+            t = fmax(t, cg::this_cluster().map_shared_rank(const_cast<double *>(part), r)[e]);
+        return t;
+    }
+    // no CTA leaves while another may still read its shared memory
+    __device__ void leave() const {
+        if (size > 1) cg::this_cluster().sync();
+    }
+};
+
+// CTAs of a team: `per` elements each, up to 16 CTAs (of one GPC: above the
+// portable 8)
+int team_size(i64 n, i64 per) {
+    int c = 1;
+    while (c < 16 && (i64)c * per < n) c *= 2;
+    return c;
 }
 
-__device__ double block_dot(const double *x, const double *y, int n, double *sh) {
-    double a = 0.0;
-    for (int k = threadIdx.x; k < n; k += DT) a = fma(x[k], y[k], a);
-    return block_sum(a, sh);
+template <class... P, class... A>
+int launch_team(void (*kern)(P...), int teams, int size, size_t smem, const char *what, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(teams * size));
+    cfg.blockDim = dim3(DT);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream();
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)size;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cuda_check(cudaLaunchKernelEx(&cfg, kern, P(args)...), what);
+}
+template <class K>
+int team_attrs(K *kern, size_t smem, std::atomic<bool> &done) {
+    if (done.load(std::memory_order_acquire)) return CPSD_OK;
+    if (smem)
+        CPSD_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                            "solver smem attr"));
+    CPSD_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                        "solver cluster attr"));
+    done.store(true, std::memory_order_release);
+    return CPSD_OK;
 }
 
 // value of the first element of largest magnitude (BLAS idamax semantics)
@@ -74,68 +140,6 @@ __device__ double block_amax(const double *x, int n, double *sh, int *shi) {
     return (idx < n) ? x[idx] : 0.0;
 }
 
-// out[r] = x_r . y_r for the nr vector pairs x_r = x + r n, y_r = y + r n,
-// each summed in block_dot's order (strided per-thread sums, warp
-// shuffle-down, warp totals in warp order), with two barriers for all r
-__device__ void block_dots(const double *x, const double *y, int n, int nr, double *red, double *out) {
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    for (int r = 0; r < nr; r++) {
-        double a = 0.0;
-        for (int k = threadIdx.x; k < n; k += DT) a = fma(x[(size_t)r * n + k], y[(size_t)r * n + k], a);
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-        if (l == 0) red[r * (DT / 32) + w] = a;
-    }
-    __syncthreads();
-    if (threadIdx.x < nr) {
-        double s = 0.0;
-        for (int i = 0; i < DT / 32; i++) s += red[threadIdx.x * (DT / 32) + i];
-        out[threadIdx.x] = s;
-    }
-    __syncthreads();
-}
-
-// out[r] = block_amax of x_r = x + r n for r < nr (value of the first
-// element of largest magnitude), with two barriers for all r
-__device__ void block_amaxs(const double *x, int n, int nr, double *redv, int *redi, double *out) {
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    for (int r = 0; r < nr; r++) {
-        double best = -1.0;
-        int bi = 0x7fffffff;
-        for (int k = threadIdx.x; k < n; k += DT) {
-            const double a = fabs(x[(size_t)r * n + k]);
-            if (a > best) {
-                best = a;
-                bi = k;
-            }
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_down_sync(0xffffffffu, best, o);
-            const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-            if (ob > best || (ob == best && oi < bi)) {
-                best = ob;
-                bi = oi;
-            }
-        }
-        if (l == 0) {
-            redv[r * (DT / 32) + w] = best;
-            redi[r * (DT / 32) + w] = bi;
-        }
-    }
-    __syncthreads();
-    if (threadIdx.x < nr) {
-        const int r = threadIdx.x;
-        double bv = -1.0;
-        int ii = 0x7fffffff;
-        for (int i = 0; i < DT / 32; i++)
-            if (redv[r * (DT / 32) + i] > bv || (redv[r * (DT / 32) + i] == bv && redi[r * (DT / 32) + i] < ii)) {
-                bv = redv[r * (DT / 32) + i];
-                ii = redi[r * (DT / 32) + i];
-            }
-        out[r] = (ii < n) ? x[(size_t)r * n + ii] : 0.0;
-    }
-    __syncthreads();
-}
-
 // dot product of two length-n vectors by one warp (result in every lane)
 __device__ double warp_dot(const double *x, const double *y, int n) {
     const int lane = threadIdx.x & 31;
@@ -146,16 +150,17 @@ __device__ double warp_dot(const double *x, const double *y, int n) {
     return a;
 }
 
-// Cyclic Jacobi on the symmetric n x n matrix S (row-major, ld DAV_MAXD,
-// zero outside n x n) by the whole block; eigenvectors accumulate in the
-// columns of V.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an
-// element with a_pq^2 <= 1e-34 |a_pp a_qq| is negligible and set to zero; a
-// sweep without rotations ends the iteration.  The n(n-1)/2 rotations of a
-// sweep run as n-1 rounds of n/2 disjoint rotations (round-robin pairing,
-// n padded to even), each round one parallel update of S and V.  The
-// iteration ends at the first round whose matrix has no element above the
-// threshold: the rounds left of that sweep and the sweep without rotations
-// would change no diagonal element and no column of V.  The
+constexpr int GL = DAV_MAXD + 1;
+
+// Cyclic Jacobi on the symmetric n x n matrix in S (ld GL, zero outside
+// n x n) by the whole block; the eigenvalues end on the diagonal of S, the
+// eigenvectors in the columns of V (ld GL).  S2 and V2 are scratch of the
+// same size.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an element
+// with a_pq^2 <= 1e-34 |a_pp a_qq| is negligible and set to zero.  The
+// n(n-1)/2 rotations of a sweep run as n-1 rounds of n/2 disjoint rotations
+// (round-robin pairing, n padded to even), each round one parallel update of
+// S and V.  The iteration ends at the first round whose matrix has no
+// element above the threshold: later rounds would change nothing.  The
 // rotation of a pair is the smaller root t of t^2 + 2 tau t - 1 = 0, tau =
 // d / b, d = a_qq - a_pp, b = 2 a_pq, by its half angle:
 //   h = 1 / sqrt(d^2 + b^2),  u = (1 + |d| h) / 2,  r = 1 / sqrt(u),
@@ -164,29 +169,44 @@ __device__ double warp_dot(const double *x, const double *y, int n) {
 // d^2 + b^2 leaves the normal range is scaled first.
 //
 // Latency bounds it: about 80 rounds at n = 20, each a chain of the rotation
-// parameters, two block barriers and one 2 x 2 update.  So each thread's
-// elements of the test, the update and V are worked out once, before the
-// rounds, and the test squares instead of taking roots.
-__device__ void block_jacobi(double *S, double *V, int n) {
-    __shared__ double cs[DAV_MAXD], sn[DAV_MAXD];
+// parameters, a barrier, one 2 x 2 update and a barrier.  So pair k always
+// sits in rows and columns 2k and 2k + 1 and the update writes to the places
+// of the next round's pairing, in the other of two buffers: every address of
+// a thread is the same in all rounds.  (Indexing the pairs anew took 1250
+// cycles a round; roots, divisions and the index arithmetic 2000.)
+__device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n) {
+    __shared__ double cs[DAV_MAXD / 2], sn[DAV_MAXD / 2];
+    __shared__ int rotate;  // last round that saw an element above the threshold
     const int tid = threadIdx.x;
     const int m = (n + 1) & ~1, half = m / 2;
     for (int e = tid; e < DAV_MAXD * DAV_MAXD; e += DT) {
-        int i = e / DAV_MAXD, j = e % DAV_MAXD;
-        V[e] = (i == j && i < m) ? 1.0 : 0.0;
+        const int i = e / DAV_MAXD, j = e % DAV_MAXD;
+        V[i * GL + j] = (i == j && i < m) ? 1.0 : 0.0;
+        V2[i * GL + j] = 0.0;
     }
-    // this thread's elements p < q of the threshold test (warps 1..: at most
-    // two of the 496), numbered by columns
-    int tp[2] = {-1, -1}, tq[2] = {0, 0};
+    if (tid == 0) rotate = 0;
+    // round robin: the players of a circle move one place on, the one at
+    // place 0 stays; place 2k faces 2k + 1
+    auto next = [&](int i) {
+        if (i == 0 || m == 2) return i;
+        if (i == m - 2) return m - 1;           // end of the upper row turns back
+        if ((i & 1) == 0) return i + 2;         // upper row moves out
+        return i == 1 ? 2 : i - 2;              // lower row moves in
+    };
+    // this thread's elements i < j of the threshold test (warps 1..: at most
+    // two of the 496), numbered along the rows
+    int to[2] = {-1, -1}, tp[2] = {0, 0}, tq[2] = {0, 0};
     if (tid >= 32)
 #pragma unroll
         for (int w = 0; w < 2; w++) {
-            const int e = tid - 32 + w * (DT - 32);
-            if (e < n * (n - 1) / 2) {
-                int q = 1;
-                while ((q + 1) * q / 2 <= e) q++;
-                tp[w] = e - q * (q - 1) / 2;
-                tq[w] = q;
+            int e = tid - 32 + w * (DT - 32);
+            if (e < m * (m - 1) / 2) {
+                int i = 0;
+                while (e >= m - 1 - i) e -= m - 1 - i++;
+                const int j = i + 1 + e;
+                to[w] = i * GL + j;
+                tp[w] = i * (GL + 1);
+                tq[w] = j * (GL + 1);
             }
         }
     // its 2 x 2 block (pair k rows, pair l columns) of S (first half of the
@@ -196,93 +216,115 @@ __device__ void block_jacobi(double *S, double *V, int n) {
     const int k0 = e0 / half, l0 = e0 - k0 * half;
     const int e1 = e0 + DT / 2, k1 = e1 / half, l1 = e1 - k1 * half;
     const bool live0 = on_s ? k0 < half : k0 < m, live1 = !on_s && k1 < m;
-    // the pair of index k in round r: (r, m-1) for k = 0, else r + k and r - k
-    // modulo m-1; smaller one first
-    auto pair_of = [&](int k, int r, int *p, int *q) {
-        int a = r + k, b = r - k;
-        if (a >= m - 1) a -= m - 1;
-        if (b < 0) b += m - 1;
-        if (k == 0) b = m - 1;
-        *p = min(a, b);
-        *q = max(a, b);
-    };
-    __syncthreads();
-    bool done = m <= 1;
-    for (int sweep = 0; sweep < 50 && !done; sweep++) {
-        for (int r = 0; r < m - 1; r++) {
-            // does any element of the matrix still call for a rotation?
-            // (asked by warps 1.., beside warp 0's rotation parameters)
-            bool above = false;
-#pragma unroll
-            for (int w = 0; w < 2; w++)
-                if (tp[w] >= 0) {
-                    const double apq = S[tp[w] * DAV_MAXD + tq[w]];
-                    above |= !(apq * apq <= 1.0e-34 * fabs(S[tp[w] * (DAV_MAXD + 1)] * S[tq[w] * (DAV_MAXD + 1)]) ||
-                               apq == 0.0);
-                }
-            if (tid < half) {
-                int p, q;
-                pair_of(tid, r, &p, &q);
-                const double apq = S[p * DAV_MAXD + q];
-                const double app = S[p * DAV_MAXD + p], aqq = S[q * DAV_MAXD + q];
-                double c = 1.0, s = 0.0;
-                if (!(apq * apq <= 1.0e-34 * fabs(app * aqq) || apq == 0.0)) {
-                    double d = aqq - app, b = 2.0 * apq, h2 = fma(d, d, b * b);
-                    if (!(h2 > 1.0e-290 && h2 < 1.0e290)) {
-                        const double f = 1.0 / fmax(fabs(d), fabs(b));
-                        d *= f;
-                        b *= f;
-                        h2 = fma(d, d, b * b);
-                    }
-                    const double h = rsqrt(h2), u = fma(0.5 * fabs(d), h, 0.5), ru = rsqrt(u);
-                    c = u * ru;
-                    s = 0.5 * fabs(b) * h * ru;
-                    if (d != 0.0 && ((d > 0.0) != (b > 0.0))) s = -s;
-                }
-                cs[tid] = c;
-                sn[tid] = s;
-            }
-            if (!__syncthreads_or(above)) {
-                done = true;
-                break;
-            }
-            // S <- J^T S J on the 2x2 blocks, V <- V J
-            if (on_s) {
-                if (live0) {
-                    int pk, qk, pl, ql;
-                    pair_of(k0, r, &pk, &qk);
-                    pair_of(l0, r, &pl, &ql);
-                    const double ck = cs[k0], sk = sn[k0], cl = cs[l0], sl = sn[l0];
-                    const double b00 = S[pk * DAV_MAXD + pl], b01 = S[pk * DAV_MAXD + ql];
-                    const double b10 = S[qk * DAV_MAXD + pl], b11 = S[qk * DAV_MAXD + ql];
-                    const double t00 = cl * b00 - sl * b01, t01 = sl * b00 + cl * b01;
-                    const double t10 = cl * b10 - sl * b11, t11 = sl * b10 + cl * b11;
-                    const bool dia = k0 == l0;  // annihilated (or negligible) element
-                    S[pk * DAV_MAXD + pl] = ck * t00 - sk * t10;
-                    S[pk * DAV_MAXD + ql] = dia ? 0.0 : ck * t01 - sk * t11;
-                    S[qk * DAV_MAXD + pl] = dia ? 0.0 : sk * t00 + ck * t10;
-                    S[qk * DAV_MAXD + ql] = sk * t01 + ck * t11;
-                }
-            } else {
-                if (live0) {
-                    int p, q;
-                    pair_of(l0, r, &p, &q);
-                    const double c = cs[l0], s = sn[l0], vp = V[k0 * DAV_MAXD + p], vq = V[k0 * DAV_MAXD + q];
-                    V[k0 * DAV_MAXD + p] = c * vp - s * vq;
-                    V[k0 * DAV_MAXD + q] = s * vp + c * vq;
-                }
-                if (live1) {
-                    int p, q;
-                    pair_of(l1, r, &p, &q);
-                    const double c = cs[l1], s = sn[l1], vp = V[k1 * DAV_MAXD + p], vq = V[k1 * DAV_MAXD + q];
-                    V[k1 * DAV_MAXD + p] = c * vp - s * vq;
-                    V[k1 * DAV_MAXD + q] = s * vp + c * vq;
-                }
-            }
-            __syncthreads();
-        }
+    const int cp = next(2 * l0), cq = next(2 * l0 + 1);
+    int r0, r1, w00, w01, w10, w11;
+    if (on_s) {
+        r0 = 2 * k0 * GL + 2 * l0;
+        r1 = r0 + GL;
+        w00 = next(2 * k0) * GL + cp;
+        w01 = next(2 * k0) * GL + cq;
+        w10 = next(2 * k0 + 1) * GL + cp;
+        w11 = next(2 * k0 + 1) * GL + cq;
+    } else {
+        r0 = k0 * GL + 2 * l0;
+        r1 = k1 * GL + 2 * l1;
+        w00 = k0 * GL + cp;
+        w01 = k0 * GL + cq;
+        w10 = k1 * GL + next(2 * l1);
+        w11 = k1 * GL + next(2 * l1 + 1);
     }
+    const bool dia = on_s && k0 == l0;
+    double *A = S, *B = S2, *E = V, *F = V2;
     __syncthreads();
+    for (int round = 1; round <= 50 * (m - 1); round++) {
+        // does any element of the matrix still call for a rotation?
+        // (asked by warps 1.., beside warp 0's rotation parameters)
+        bool above = false;
+#pragma unroll
+        for (int w = 0; w < 2; w++)
+            if (to[w] >= 0) {
+                const double x = A[to[w]];
+                above |= !(x * x <= 1.0e-34 * fabs(A[tp[w]] * A[tq[w]]) || x == 0.0);
+            }
+        if (above) rotate = round;
+        const double *src = on_s ? A : E;
+        double b00 = 0.0, b01 = 0.0, b10 = 0.0, b11 = 0.0;
+        if (live0) {
+            b00 = src[r0];
+            b01 = src[r0 + 1];
+        }
+        if (on_s ? live0 : live1) {
+            b10 = src[r1];
+            b11 = src[r1 + 1];
+        }
+        if (tid < half) {
+            const int o = 2 * tid * (GL + 1);
+            const double app = A[o], aqq = A[o + GL + 1], apq = A[o + 1];
+            double d = aqq - app, b = 2.0 * apq, h2 = fma(d, d, b * b);
+            const bool keep = apq * apq <= 1.0e-34 * fabs(app * aqq) || apq == 0.0;
+            if (!keep && !(h2 > 1.0e-290 && h2 < 1.0e290)) {
+                const double f = 1.0 / fmax(fabs(d), fabs(b));
+                d *= f;
+                b *= f;
+                h2 = fma(d, d, b * b);
+            }
+            const double h = rsqrt(h2), u = fma(0.5 * fabs(d), h, 0.5), ru = rsqrt(u);
+            double s = 0.5 * fabs(b) * h * ru;
+            if (d != 0.0 && ((d > 0.0) != (b > 0.0))) s = -s;
+            cs[tid] = keep ? 1.0 : u * ru;
+            sn[tid] = keep ? 0.0 : s;
+        }
+        __syncthreads();
+        if (rotate != round) break;
+        // S <- J^T S J on the 2x2 blocks, V <- V J
+        const double cl = cs[l0 < half ? l0 : 0], sl = sn[l0 < half ? l0 : 0];
+        if (on_s) {
+            if (live0) {
+                const double ck = cs[k0], sk = sn[k0];
+                const double t00 = cl * b00 - sl * b01, t01 = sl * b00 + cl * b01;
+                const double t10 = cl * b10 - sl * b11, t11 = sl * b10 + cl * b11;
+                B[w00] = ck * t00 - sk * t10;
+                B[w01] = dia ? 0.0 : ck * t01 - sk * t11;  // annihilated (or negligible) element
+                B[w10] = dia ? 0.0 : sk * t00 + ck * t10;
+                B[w11] = sk * t01 + ck * t11;
+            }
+        } else {
+            if (live0) {
+                F[w00] = cl * b00 - sl * b01;
+                F[w01] = sl * b00 + cl * b01;
+            }
+            if (live1) {
+                const double c = cs[l1], s = sn[l1];
+                F[w10] = c * b10 - s * b11;
+                F[w11] = s * b10 + c * b11;
+            }
+        }
+        double *x = A;
+        A = B;
+        B = x;
+        x = E;
+        E = F;
+        F = x;
+        __syncthreads();
+    }
+    // the padding of an odd n sits at place p: it goes last
+    if (A != S)
+        for (int e = tid; e < m * m; e += DT) {
+            const int i = e / m, j = e % m;
+            S[i * GL + j] = A[i * GL + j];
+            V[i * GL + j] = E[i * GL + j];
+        }
+    __syncthreads();
+    if (m > n) {
+        __shared__ int pad;
+        if (tid < m && V[n * GL + tid] == 1.0) pad = tid;
+        __syncthreads();
+        if (pad != n) {
+            if (tid == 0) S[pad * (GL + 1)] = S[n * (GL + 1)];
+            if (tid < m) V[tid * GL + pad] = V[tid * GL + n];
+        }
+        __syncthreads();
+    }
 }
 
 // ------------------------------------------------ general real eigenproblem
@@ -306,10 +348,9 @@ __device__ void block_jacobi(double *S, double *V, int n) {
 // control flow (deflation tests, shifts and reflectors are computed from
 // shared values by all lanes alike).  H, Z and X are row-major with leading
 // dimension GL (odd, so that a lane per row hits distinct banks); H is
-// destroyed, Z and X are scratch, V (leading dimension DAV_MAXD, may alias
-// Z) receives the vectors.  Returns the number of QR sweeps, or -1 when a
+// destroyed, Z and X are scratch, V (leading dimension GL, may alias Z)
+// receives the vectors.  Returns the number of QR sweeps, or -1 when a
 // window did not converge within 30 max(10, n) sweeps.
-constexpr int GL = DAV_MAXD + 1;
 
 __device__ __forceinline__ double warp_allsum(double v) {
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -640,40 +681,41 @@ __device__ int warp_geev(double *H, double *Z, double *X, double *V, double *wr,
     __syncwarp();
     // each column to unit norm where it is off by more than 1e-10, as the
     // reference does with the real and imaginary parts it keeps
-    // (mod_davidson.f90:211-217); copy out with V's leading dimension
+    // (mod_davidson.f90:211-217)
     if (lane < n) {
         double s = 0.0;
         for (int i = 0; i < n; i++) s += H[i * GL + lane] * H[i * GL + lane];
         const double t = sqrt(s), f = (fabs(t - 1.0) > 1.0e-10) ? 1.0 / t : 1.0;
-        for (int i = 0; i < DAV_MAXD; i++) V[i * DAV_MAXD + lane] = (i < n) ? H[i * GL + lane] * f : 0.0;
+        for (int i = 0; i < DAV_MAXD; i++) V[i * GL + lane] = (i < n) ? H[i * GL + lane] * f : 0.0;
     } else {
-        for (int i = 0; i < DAV_MAXD; i++) V[i * DAV_MAXD + lane] = 0.0;
+        for (int i = 0; i < DAV_MAXD; i++) V[i * GL + lane] = 0.0;
     }
     __syncwarp();
     return sweeps;
 }
 
 // Schmidt_2D (mod_davidson.f90:642-680) on the dim columns (length len <= 32)
-// of `in`, by one warp: lane k holds row k; modified Gram-Schmidt in the
-// reference's order
-__device__ void warp_schmidt_2d(const double *in, double *out, int len, int dim) {
-    const int lane = threadIdx.x & 31;
-    for (int i = 0; i < dim; i++)
-        if (lane < len) out[i * len + lane] = in[i * len + lane];
-    __syncwarp();
-    for (int i = 1; i < dim; i++) {
-        double x = (lane < len) ? out[i * len + lane] : 0.0;
-        for (int j = 0; j < i; j++) {
-            double y = (lane < len) ? out[j * len + lane] : 0.0;
-            double ov = x * y;
-            for (int o = 16; o > 0; o >>= 1) ov += __shfl_xor_sync(0xffffffffu, ov, o);
-            x += -ov * y;
+// of v (leading dimension GL), in place by the whole block: modified
+// Gram-Schmidt, each column projected on the earlier ones in the reference's
+// order; a warp per later column takes out column j as soon as it is final
+__device__ void block_schmidt_2d(double *v, int len, int dim) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int j = 0; j < dim; j++) {
+        if (j > 0) {
+            if (w == 0) {
+                const double x = lane < len ? v[j * GL + lane] : 0.0;
+                const double nrm = sqrt(warp_allsum(x * x));
+                if (lane < len) v[j * GL + lane] = x * (1.0 / nrm);
+            }
+            __syncthreads();
         }
-        double nrm = x * x;
-        for (int o = 16; o > 0; o >>= 1) nrm += __shfl_xor_sync(0xffffffffu, nrm, o);
-        nrm = sqrt(nrm);
-        if (lane < len) out[i * len + lane] = x * (1.0 / nrm);
-        __syncwarp();
+        const double y = lane < len ? v[j * GL + lane] : 0.0;
+        for (int i = j + 1 + w; i < dim; i += DT / 32) {
+            const double x = lane < len ? v[i * GL + lane] : 0.0;
+            const double ov = warp_allsum(x * y);
+            if (lane < len) v[i * GL + lane] = x + -ov * y;
+        }
+        __syncthreads();
     }
 }
 
@@ -686,10 +728,7 @@ __global__ void __launch_bounds__(DT) k_dav_init(DavState *st, DavBuffers b) {
         if ((threadIdx.x & 31) == 0) s.Abar[j + i * D] = v;
     }
     if (threadIdx.x == 0) {
-        for (int i = 0; i < nr; i++) {
-            s.eigenVal[i] = b.fileEV[(size_t)i * (n + 1)];
-            for (int k = 0; k < D; k++) s.vecNeed[k + i * D] = (k == i) ? 1.0 : 0.0;
-        }
+        for (int i = 0; i < nr; i++) s.eigenVal[i] = b.fileEV[(size_t)i * (n + 1)];
         s.iterations = 1;
         s.dimIter = nr;
         s.dimFree = D - nr;
@@ -697,28 +736,184 @@ __global__ void __launch_bounds__(DT) k_dav_init(DavState *st, DavBuffers b) {
         s.cur = 0;
         s.done = 0;
         s.converged = 0;
+        s.pending = 0;
     }
 }
 
-__global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b) {
-    __shared__ double S[DAV_MAXD * GL], V[DAV_MAXD * GL], X[DAV_MAXD * GL], ovl[DAV_MAXD];
-    __shared__ double sh[DT / 32 + 1];
+// Shared memory of a Davidson step.  S, X and V hold the Ritz problem, then S
+// the collapse coefficients; ex is the double-buffered exchange of a step's
+// partial sums (overlaps with the basis and Gram matrix of the new vectors,
+// or the collapsed Ritz matrix), tot their sums over the CTAs.
+constexpr int DAV_EX = 2 * DAV_MAXD * DAV_MAXD;
+constexpr int DOT_RT = 4;  // row tiles of eight vectors per pass of the products
+struct DavShared {
+    double S[DAV_MAXD * GL], V[DAV_MAXD * GL], X[DAV_MAXD * GL];
+    double ex[2][DAV_EX], tot[DAV_EX];
+    double red[DT / 32][DOT_RT * 64];  // one pass's products of each warp
+    double L[DAV_MAXD * GL];           // Cholesky factor of the new vectors
+    double2 cf[DAV_MAXD][4];           // coefficients of eight outputs
+    double vR[DAV_MAXD], vI[DAV_MAXD], ev[DAV_MAXD], rnorm[DAV_MAXD];
+    int lw[DAV_MAXD], act[DAV_MAXD], cvd[DAV_MAXD];
+    int general, eig_fail, warn, nnew;
+};
+
+// The basis, its sigma vectors and the work vectors of a step live in shared
+// memory when this many doubles hold a CTA's part of them (n up to about 3900
+// with 16 CTAs, a basis of 20 and 5 roots): copied there while the Ritz
+// problem is solved, they cost one latency instead of one for each of the
+// step's eight passes.
+constexpr int DAV_LOCAL = 13312;
+// elements a CTA, up to 16 CTAs: n = 858, 5 roots, 94 us a step at 112, 100 at
+// 224, 111 at 448 (150 on one CTA); n = 174, 3 roots, 44 us at 112, 42.5 at 224
+constexpr int DAV_PER = 192;
+// leading dimension of vectors in shared memory: 4 mod 16, so that 8 vectors
+// by 4 elements fall on different banks
+__host__ __device__ constexpr int dav_ld(int nc) { return (nc + 11) / 16 * 16 + 4; }
+
+__device__ __forceinline__ void cp_async8(double *dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// coefficients c(i, r0 + q), q < 8, of nb vectors into cf (zero past nr)
+template <class F>
+__device__ void put_coefs(double2 (*cf)[4], int nb, int r0, int nr, F coef) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < nb * 8; e += DT) {
+        const int i = e >> 3, q = e & 7;
+        reinterpret_cast<double *>(cf[i])[q] = r0 + q < nr ? coef(i, r0 + q) : 0.0;
+    }
+    __syncthreads();
+}
+
+// out(r, k, sum_i c(i, r) x_i[k], sum_i c(i, r) y_i[k]) for r < nr and the nc
+// elements k of this CTA, 8 outputs a pass so that every x_i, y_i is loaded
+// once for them (sums in basis order); the coefficients are read as pairs, a
+// broadcast of four loads a basis vector
+template <class F, class G>
+__device__ void combine(double2 (*cf)[4], int nc, int nb, int nr, const double *x, const double *y, i64 ld, F coef,
+                        G out) {
+    for (int r0 = 0; r0 < nr; r0 += 8) {
+        put_coefs(cf, nb, r0, nr, coef);
+        for (int k = threadIdx.x; k < nc; k += DT) {
+            double a[8], c[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) a[q] = c[q] = 0.0;
+#pragma unroll 4
+            for (int i = 0; i < nb; i++) {
+                const double u = x[i * ld + k], v = y[i * ld + k];
+#pragma unroll
+                for (int q = 0; q < 4; q++) {
+                    const double2 f = cf[i][q];
+                    a[2 * q] += f.x * u;
+                    a[2 * q + 1] += f.y * u;
+                    c[2 * q] += f.x * v;
+                    c[2 * q + 1] += f.y * v;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (r0 + q < nr) out(r0 + q, k, a[q], c[q]);
+        }
+    }
+}
+
+__device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// part[i * nw + q] = x_i . w_act[q] over this CTA's elements for i < nx and,
+// with gram, part[(nx + p) * nw + q] = w_act[p] . w_act[q].  FP64 tensor
+// instructions: a warp takes every 16th group of 8 elements, tiles of 8
+// vectors by 8; so each vector is read once for eight products.  Ends with a
+// block barrier.
+__device__ void team_dots(DavShared &sm, int nc, const double *x, i64 ldx, int nx, const double *w, i64 ldw,
+                          const int *act, int nw, bool gram, double *part) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, c = lane & 3;
+    const int rows = nx + (gram ? nw : 0);
+    for (int q0 = 0; q0 < nw; q0 += 8) {
+        const double *wp = q0 + g < nw ? w + act[q0 + g] * ldw : nullptr;
+        for (int i0 = 0; i0 < rows; i0 += 8 * DOT_RT) {
+            const double *xp[DOT_RT];
+            double acc[DOT_RT][2];
+#pragma unroll
+            for (int r = 0; r < DOT_RT; r++) {
+                const int i = i0 + 8 * r + g;
+                xp[r] = i < nx ? x + i * ldx : i < rows ? w + act[i - nx] * ldw : nullptr;
+                acc[r][0] = acc[r][1] = 0.0;
+            }
+            const int nt = min(DOT_RT, (rows - i0 + 7) / 8);
+#pragma unroll 2
+            for (int k = 8 * warp; k < nc; k += 8 * (DT / 32)) {
+                const int ka = k + c, kb = ka + 4;
+                const double ba = wp && ka < nc ? wp[ka] : 0.0, bb = wp && kb < nc ? wp[kb] : 0.0;
+                double aa[DOT_RT], ab[DOT_RT];
+#pragma unroll
+                for (int r = 0; r < DOT_RT; r++) {
+                    aa[r] = xp[r] && ka < nc ? xp[r][ka] : 0.0;
+                    ab[r] = xp[r] && kb < nc ? xp[r][kb] : 0.0;
+                }
+#pragma unroll
+                for (int r = 0; r < DOT_RT; r++)
+                    if (r < nt) {
+                        dmma884(acc[r], aa[r], ba);
+                        dmma884(acc[r], ab[r], bb);
+                    }
+            }
+#pragma unroll
+            for (int r = 0; r < DOT_RT; r++)
+                if (r < nt)
+                    *reinterpret_cast<double2 *>(&sm.red[warp][r * 64 + g * 8 + 2 * c]) = make_double2(acc[r][0], acc[r][1]);
+            __syncthreads();
+            if ((int)threadIdx.x < nt * 64) {
+                const int i = i0 + (int)threadIdx.x / 8, q = q0 + ((int)threadIdx.x & 7);
+                if (i < rows && q < nw) {
+                    double v = 0.0;
+#pragma unroll
+                    for (int u = 0; u < DT / 32; u++) v += sm.red[u][threadIdx.x];
+                    part[i * nw + q] = v;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// One Davidson step by the CTAs of a cluster.  Latency bounds it for SF-CIS
+// (n of a few hundred), bandwidth for (R1, R2) vectors, which 16 SMs stream.
+// The CTAs meet four times a step: Ritz norms and residuals together, then
+// three times for the new vectors.
+__global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int local) {
+    extern __shared__ double dav_smem[];
+    DavShared &sm = *reinterpret_cast<DavShared *>(dav_smem);
+    double *const S = sm.S, *const V = sm.V, *const X = sm.X, *const vR = sm.vR, *const vI = sm.vI;
+    int *const lw = sm.lw;
     DavState &s = *st;
     const int tid = threadIdx.x;
     const int D = s.D, n = s.dimA, nroot = s.nroot;
     if (s.done) return;
-    if (s.iterations > s.maxcyc) {
-        if (tid == 0) {
-            s.done = 1;
-            if (b.mailbox) {
-                b.mailbox[0] = 0;
-                __threadfence_system();
-            }
+    Team t(n);
+    const int lo = t.lo, nc = t.hi - t.lo;
+    // the sigma vectors staged by the step before belong to the subspace now
+    const int iterations = s.iterations + s.pending;
+    int dimIter = s.dimIter + (s.pending ? s.nNew : 0), cur = s.cur, dimFree = s.dimFree;
+    const int dim_exceed = s.dim_exceed, ndimIter = s.ndimIter, ndimFree = s.ndimFree;
+    const bool over = iterations > s.maxcyc;
+    // this CTA's part of the vectors: x_i[k] at x[i ld + k]
+    const i64 ld = local ? dav_ld(nc) : n;
+    double *const room = dav_smem + (sizeof(DavShared) + 15) / 16 * 2;
+    double *Bl = local ? room : b.B[cur] + lo, *ABl = local ? room + D * ld : b.AB[cur] + lo;
+    double *const W0 = local ? room + 2 * D * ld : b.w0 + lo, *const W1 = local ? W0 + nroot * ld : b.w1 + lo;
+    const double dk0 = tid < nc ? b.diag[lo + tid] : 0.0;  // the first element's diagonal
+    if (local && !over)
+        for (int e = tid; e < dimIter * nc; e += DT) {
+            const int i = e / nc, k = e - i * nc;
+            cp_async8(Bl + i * ld + k, b.B[cur] + (size_t)i * n + lo + k);
+            cp_async8(ABl + i * ld + k, b.AB[cur] + (size_t)i * n + lo + k);
         }
-        return;
-    }
-    int dimIter = s.dimIter, cur = s.cur, dimFree = s.dimFree;
-    const int dim_exceed = s.dim_exceed;
+    int &general = sm.general, &eig_fail = sm.eig_fail, &warn = sm.warn;
     // ---- step 3: eigenpairs of Abar, dgeev in the reference
     // (mod_davidson.f90:185-219).  Abar = B^T A B is symmetric when A is
     // (spin-flip CIS with real integrals); when it is symmetric to 1e-12 of
@@ -726,65 +921,66 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b) {
     // dgeev's eigenpairs (to rounding) fastest; otherwise one warp solves
     // the general problem (warp_geev: real parts of the eigenvalues, real
     // and imaginary parts of complex eigenvectors as dgeev returns them,
-    // complex values counted as the reference's imaginary-eigenvalue warning)
-    __shared__ double vR[DAV_MAXD], vI[DAV_MAXD];
-    __shared__ int lw[DAV_MAXD], general;
-    if (tid < 32) {
-        double am = 0.0, ad = 0.0;
-        if (tid < dimIter)
-            for (int i = 0; i < dimIter; i++) {
-                const double aij = s.Abar[i + tid * D], aji = s.Abar[tid + i * D];
-                am = fmax(am, fabs(aij));
-                ad = fmax(ad, fabs(aij - aji));
-            }
-        am = warp_allmax(am);
-        ad = warp_allmax(ad);
-        if (tid == 0) general = ad > 1.0e-12 * am;
-    }
-    __syncthreads();
-    if (!general) {
-        for (int e = tid; e < DAV_MAXD * DAV_MAXD; e += DT) {
-            int i = e / DAV_MAXD, j = e % DAV_MAXD;
-            S[e] = (i < dimIter && j < dimIter) ? 0.5 * (s.Abar[i + j * D] + s.Abar[j + i * D]) : 0.0;
-        }
-        __syncthreads();
-        block_jacobi(S, V, dimIter);
-        if (tid < dimIter) vR[tid] = S[tid * DAV_MAXD + tid];
-    } else {
-        for (int e = tid; e < dimIter * dimIter; e += DT) {
-            const int i = e / dimIter, j = e % dimIter;
-            S[i * GL + j] = s.Abar[i + j * D];
-        }
-        __syncthreads();
+    // complex values counted as the reference's imaginary-eigenvalue
+    // warning).  Every CTA solves it for itself.
+    if (tid == 0) eig_fail = warn = 0;
+    if (!over) {
         if (tid < 32) {
-            const int sw = warp_geev(S, V, X, V, vR, vI, dimIter);
-            if (tid == 0) {
-                s.nonsym_steps++;
-                if (sw < 0) s.eig_fail = 1;
-                for (int i = 0; i < dimIter; i++)
-                    if (fabs(vI[i]) > 1.0e-10) s.warn_imag++;
+            double am = 0.0, ad = 0.0;
+            if (tid < dimIter)
+                for (int i = 0; i < dimIter; i++) {
+                    const double aij = s.Abar[i + tid * D], aji = s.Abar[tid + i * D];
+                    am = fmax(am, fabs(aij));
+                    ad = fmax(ad, fabs(aij - aji));
+                }
+            am = warp_allmax(am);
+            ad = warp_allmax(ad);
+            if (tid == 0) general = ad > 1.0e-12 * am;
+        }
+        __syncthreads();
+        if (!general) {
+            for (int e = tid; e < DAV_MAXD * DAV_MAXD; e += DT) {
+                int i = e / DAV_MAXD, j = e % DAV_MAXD;
+                S[i * GL + j] = (i < dimIter && j < dimIter) ? 0.5 * (s.Abar[i + j * D] + s.Abar[j + i * D]) : 0.0;
+            }
+            __syncthreads();
+            block_jacobi(S, V, X, sm.tot, dimIter);
+            if (tid < dimIter) vR[tid] = S[tid * GL + tid];
+        } else {
+            for (int e = tid; e < dimIter * dimIter; e += DT) {
+                const int i = e / dimIter, j = e % dimIter;
+                S[i * GL + j] = s.Abar[i + j * D];
+            }
+            __syncthreads();
+            if (tid < 32) {
+                const int sw = warp_geev(S, V, X, V, vR, vI, dimIter);
+                if (tid == 0) {
+                    eig_fail = sw < 0;
+                    warn = 0;
+                    for (int i = 0; i < dimIter; i++)
+                        if (fabs(vI[i]) > 1.0e-10) warn++;
+                }
             }
         }
     }
-    __syncthreads();
-    if (s.eig_fail) {  // the QR iteration did not converge: stop the solver
-        if (tid == 0) {
-            s.done = 1;
-            if (b.mailbox) {
-                b.mailbox[0] = 0;
-                __threadfence_system();
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    t.sync();  // every CTA has read the state
+    if (over || eig_fail) {  // cycle limit, or the QR iteration did not converge: stop the solver
+        if (t.rank == 0 && tid == 0) {
+            s.iterations = iterations;
+            s.dimIter = dimIter;
+            s.pending = 0;
+            if (eig_fail) {
+                s.eig_fail = 1;
+                s.nonsym_steps++;
+                s.warn_imag += warn;
             }
+            s.done = 1;
+            if (b.mailbox) b.mailbox[0] = 0;
         }
         return;
     }
-    // eigenvalues, their order and the chosen roots, worked out in shared
-    // memory (vecR(i, k) = V[i][k] for i < dimIter, zero below) and then
-    // published to the state
-    for (int e = tid; e < D * dimIter; e += DT) {
-        int i = e % D, k = e / D;
-        s.vecR[i + k * D] = (i < dimIter) ? V[i * DAV_MAXD + k] : 0.0;
-    }
-    __syncthreads();
+    // eigenvalues, their order and the chosen roots (vecR(i, k) = V[i][k])
     // sort (mod_davidson.f90:620-640): position = number of smaller values;
     // equal values keep the order that the reference's exchanges leave
     if (tid < 32) {
@@ -819,7 +1015,7 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b) {
         if (!s.lowest)
             for (int iroot = 0; iroot < nroot; iroot++) {
                 const int mine = tid < dimIter ? lw[tid] : 0;
-                double best = tid >= iroot && tid < dimIter ? fabs(V[iroot * DAV_MAXD + (mine - 1)]) : 0.0;
+                double best = tid >= iroot && tid < dimIter ? fabs(V[iroot * GL + (mine - 1)]) : 0.0;
                 int at = best > 0.0 ? tid : iroot;
                 if (!(best > 0.0)) best = 0.0;
                 for (int o = 16; o > 0; o >>= 1) {
@@ -838,231 +1034,367 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b) {
             }
     }
     __syncthreads();
-    if (tid < dimIter) {
-        s.valR[tid] = vR[tid];
-        s.lowestE[tid] = lw[tid];
-    }
-    if (tid < nroot) s.eigenVal[tid] = vR[lw[tid] - 1];
-    for (int e = tid; e < nroot * D; e += DT) {
-        const int ir = e / D, k = e % D;
-        s.vecNeed[k + ir * D] = (k < dimIter) ? V[k * DAV_MAXD + (lw[ir] - 1)] : 0.0;
-    }
+    if (tid < nroot) sm.ev[tid] = vR[lw[tid] - 1];
     __syncthreads();
     // ---- collapse when the subspace was full (mod_davidson.f90:266-325)
     if (dim_exceed) {
-        const int nd = s.ndimIter;
+        const int nd = ndimIter;
         for (int e = tid; e < nd * dimIter; e += DT) {
-            int k = e % dimIter, i = e / dimIter;
-            s.oldE[k + i * dimIter] = s.vecR[k + (s.lowestE[i] - 1) * D];
+            const int k = e % dimIter, i = e / dimIter;
+            S[i * GL + k] = V[k * GL + (lw[i] - 1)];
         }
+        if (tid < nd) sm.act[tid] = tid;
         __syncthreads();
-        if (tid < 32) warp_schmidt_2d(s.oldE, s.newE, dimIter, nd);
-        __syncthreads();
-        const int nw = 1 - cur;
-        for (int ir = 0; ir < nd; ir++)
-            for (int k = tid; k < n; k += DT) {
-                double a = 0.0, c = 0.0;
-                for (int i = 0; i < dimIter; i++) {
-                    double t = s.newE[i + ir * dimIter];
-                    a += t * b.AB[cur][(size_t)i * n + k];
-                    c += t * b.B[cur][(size_t)i * n + k];
-                }
-                b.AB[nw][(size_t)ir * n + k] = a;
-                b.B[nw][(size_t)ir * n + k] = c;
+        block_schmidt_2d(S, dimIter, nd);
+        cur = 1 - cur;
+        double *const gB = b.B[cur] + lo, *const gAB = b.AB[cur] + lo;
+        // in shared memory an element's new values replace the old ones once
+        // all of them are formed
+        if (local && nd > 8) {
+            for (int r0 = 0; r0 < nd; r0 += 8) {
+                combine(sm.cf, nc, dimIter, min(8, nd - r0), ABl, Bl, ld,
+                        [&](int i, int r) { return S[(r0 + r) * GL + i]; },
+                        [&](int r, int k, double x, double y) {
+                            gAB[(size_t)(r0 + r) * n + k] = x;
+                            gB[(size_t)(r0 + r) * n + k] = y;
+                        });
             }
-        __syncthreads();
-        cur = nw;
-        dimFree = s.ndimFree;
-        dimIter = nd;
-        for (int e = tid >> 5; e < dimIter * dimIter; e += DT / 32) {
-            const int i = e / dimIter, j = e % dimIter;
-            double v = warp_dot(b.AB[cur] + (size_t)i * n, b.B[cur] + (size_t)j * n, n);
-            if ((tid & 31) == 0) s.Abar[j + i * D] = v;
+            __syncthreads();
+            for (int e = tid; e < nd * nc; e += DT) {
+                const int i = e / nc, k = e - i * nc;
+                ABl[i * ld + k] = gAB[(size_t)i * n + k];
+                Bl[i * ld + k] = gB[(size_t)i * n + k];
+            }
+        } else {
+            combine(sm.cf, nc, dimIter, nd, ABl, Bl, ld, [&](int i, int r) { return S[r * GL + i]; },
+                    [&](int r, int k, double x, double y) {
+                        gAB[(size_t)r * n + k] = x;
+                        gB[(size_t)r * n + k] = y;
+                        if (local) {
+                            ABl[r * ld + k] = x;
+                            Bl[r * ld + k] = y;
+                        }
+                    });
+            if (!local) {
+                ABl = gAB;
+                Bl = gB;
+            }
         }
         __syncthreads();
+        dimFree = ndimFree;
+        dimIter = nd;
+        double *part = t.next(sm.ex[0], DAV_EX);
+        team_dots(sm, nc, ABl, ld, nd, Bl, ld, sm.act, nd, false, part);
+        t.sync();
+        if (t.rank == 0)
+            for (int e = tid; e < nd * nd; e += DT) s.Abar[e % nd + (e / nd) * D] = t.sum(part, e);
     }
     // ---- steps 4-6.  The Ritz vector, residual, convergence test and
     // preconditioned vector of a root depend only on the subspace before this
     // step (the new vectors go to positions >= dimIter), so they are formed
-    // for all roots at once in per-root slices of w0 / w1 (each reduction
-    // summed in block_dot / block_amax order); only the Schmidt projections
-    // and the insertion of the new vectors run root after root.
-    __shared__ double rd[DAV_MAXD * (DT / 32)], rv[DAV_MAXD];
-    __shared__ int ri[DAV_MAXD * (DT / 32)], cvd[DAV_MAXD];
-    double *const W0 = b.w0, *const W1 = b.w1;
+    // for all roots at once in per-root slices of w0 / w1.  The norm t of a
+    // Ritz vector q and the largest element of A q - w q are found in one
+    // pass: where t is off 1 by more than 1e-10, both are divided by it.
     if (dim_exceed) {
-        for (int e = tid; e < nroot * n; e += DT) {
-            const int ir = e / n, k = e - ir * n;
-            W0[(size_t)ir * n + k] = b.AB[cur][(size_t)ir * n + k];
-            W1[(size_t)ir * n + k] = b.B[cur][(size_t)ir * n + k];
-        }
+        for (int ir = 0; ir < nroot; ir++)
+            for (int k = tid; k < nc; k += DT) {
+                W0[ir * ld + k] = ABl[ir * ld + k];
+                W1[ir * ld + k] = Bl[ir * ld + k];
+            }
     } else {
-        // one pass over the basis serves RB roots: element k of every basis
-        // vector is loaded once and summed into each root in basis order
-        // (coefficient vecNeed(i, root) = V[i][lw[root] - 1])
-        constexpr int RB = 8;
-        for (int r0 = 0; r0 < nroot; r0 += RB) {
-            const int nr = min(RB, nroot - r0);
-            int col[RB];
+        combine(sm.cf, nc, dimIter, nroot, ABl, Bl, ld, [&](int i, int r) { return V[i * GL + (lw[r] - 1)]; },
+                [&](int r, int k, double x, double y) {
+                    W0[r * ld + k] = x;
+                    W1[r * ld + k] = y;
+                });
+    }
+    {
+        const int w = tid >> 5;
+        double *const rq = sm.red[0], *const rb = rq + DT;  // [root][warp]
+        for (int r0 = 0; r0 < nroot; r0 += 4) {  // a thread's own elements: no barrier needed
+            double q2[4], big[4];
 #pragma unroll
-            for (int q = 0; q < RB; q++) col[q] = q < nr ? lw[r0 + q] - 1 : 0;
-            for (int k = tid; k < n; k += DT) {
-                double a[RB], c[RB];
+            for (int u = 0; u < 4; u++) {
+                const int ir = min(r0 + u, nroot - 1);
+                const double ev = sm.ev[ir];
+                q2[u] = 0.0;
+                big[u] = -1.0;
+                for (int k = tid; k < nc; k += DT) {
+                    const double q = W1[ir * ld + k], a = fabs(W0[ir * ld + k] - ev * q);
+                    q2[u] = fma(q, q, q2[u]);
+                    if (a > big[u]) big[u] = a;
+                }
+            }
 #pragma unroll
-                for (int q = 0; q < RB; q++) a[q] = c[q] = 0.0;
+            for (int u = 0; u < 4; u++) {
+                q2[u] = warp_allsum(q2[u]);
+                big[u] = warp_allmax(big[u]);
+            }
+            if ((tid & 31) == 0)
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if (r0 + u < nroot) {
+                        rq[(r0 + u) * (DT / 32) + w] = q2[u];
+                        rb[(r0 + u) * (DT / 32) + w] = big[u];
+                    }
+        }
+        __syncthreads();
+        double *part = t.next(sm.ex[0], DAV_EX);
+        if (tid < nroot) {
+            double q2 = 0.0, big = -1.0;
+            for (int i = 0; i < DT / 32; i++) {
+                q2 += rq[tid * (DT / 32) + i];
+                big = fmax(big, rb[tid * (DT / 32) + i]);
+            }
+            part[tid] = q2;
+            part[DAV_MAXD + tid] = big;
+        }
+        t.sync();
+        if (tid < nroot) {
+            const double nrm = sqrt(t.sum(part, tid)), big = t.amax(part, DAV_MAXD + tid);
+            const double f = fabs(nrm - 1.0) > 1.0e-10 ? 1.0 / nrm : 1.0;
+            sm.rnorm[tid] = f;
+            sm.cvd[tid] = (big >= 0.0 ? big * f : 0.0) < s.maxError ? 1 : 0;
+        }
+        __syncthreads();
+    }
+    int nconv = 0, na = 0;  // na: roots that get a new vector
+    for (int ir = 0; ir < nroot; ir++) nconv += sm.cvd[ir];
+    if (dimFree > 0)
+        for (int ir = 0; ir < nroot; ir++) {
+            if (sm.cvd[ir]) continue;
+            if (tid == 0) sm.act[na] = ir;
+            na++;
+        }
+    for (int k = tid; k < nc; k += DT) {
+        const double dk = k == tid ? dk0 : b.diag[lo + k];
+#pragma unroll 4
+        for (int ir = 0; ir < nroot; ir++) {
+            const double f = sm.rnorm[ir], ev = sm.ev[ir];
+            const double q = W1[ir * ld + k] * f, r = W0[ir * ld + k] * f - ev * q;
+            b.fileEV[(size_t)ir * (n + 1) + 1 + lo + k] = q;
+            double d = ev - dk;
+            if (fabs(d) < 1.0e-4) d = (d < 0.0) ? -1.0e-4 : 1.0e-4;
+            if (!sm.cvd[ir]) W1[ir * ld + k] = r / d;
+        }
+    }
+    __syncthreads();
+    // SchmidtS (mod_davidson.f90:682-727) of all new vectors together: twice
+    // projected on the basis (overlaps of a pass computed at once, as
+    // classical Gram-Schmidt applied twice), then made orthonormal among
+    // themselves in root order by the Cholesky factor of their Gram matrix,
+    // a vector that keeps less than 1e-6 of its length being dropped; one
+    // more pass of both takes out what the divisions by those lengths
+    // amplified.  Same vectors as the reference's one-by-one projections, to
+    // rounding, with three exchanges instead of five for every root.
+    int nNew = 0;
+    for (int pass = 0; pass < 3 && na > 0; pass++) {
+        // pass 0: overlaps and lengths; 1, 2: overlaps and Gram matrix
+        double *part = t.next(sm.ex[0], DAV_EX);
+        team_dots(sm, nc, Bl, ld, dimIter, W1, ld, sm.act, na, true, part);
+        t.sync();
+        const int no = dimIter * na;
+        for (int e = tid; e < no + na * na; e += DT) sm.tot[e] = t.sum(part, e);
+        __syncthreads();
+        if (pass > 0) {  // Gram matrix less the projections
+            for (int e = tid; e < na * na; e += DT) {
+                const int q = e / na, p = e - q * na;
+                double g = sm.tot[no + e];
+#pragma unroll 4
+                for (int i = 0; i < dimIter; i++) g -= sm.tot[i * na + q] * sm.tot[i * na + p];
+                sm.L[q * GL + p] = g;
+            }
+            __syncthreads();
+        }
+        if (tid < 32) {
+            double *const L = sm.L;  // L(q, p) at [q * GL + p]
+            if (pass == 0) {
+                // reciprocal lengths only: the vectors are scaled to unit length
+                for (int e = tid; e < na * na; e += 32) L[(e / na) * GL + e % na] = 0.0;
+                __syncwarp();
+                if (tid < na) L[tid * GL + tid] = 1.0 / sqrt(sm.tot[no + tid * na + tid]);
+                if (tid == 0) sm.nnew = na;
+            } else {
+                // Cholesky factor column by column (lane = row); the
+                // reciprocal diagonal is kept, zero for a dropped vector
+                int kept = 0;
+                for (int p = 0; p < na; p++) {
+                    const double g = L[p * GL + p], nrm = sqrt(fmax(g, 0.0));
+                    const bool keep = !(nrm < (pass == 1 ? 1.0e-6 : 0.0)) && (pass == 2 || kept < dimFree);
+                    const double ri = keep ? 1.0 / nrm : 0.0;
+                    __syncwarp();
+                    if (tid == p) L[p * GL + p] = ri;
+                    double lqp = 0.0;
+                    if (tid > p && tid < na) {
+                        lqp = L[tid * GL + p] * ri;
+                        L[tid * GL + p] = lqp;
+                    }
+                    __syncwarp();
+                    if (tid > p && tid < na)
+                        for (int q = p + 1; q <= tid; q++) L[tid * GL + q] -= lqp * L[q * GL + p];
+                    __syncwarp();
+                    kept += keep;
+                }
+                if (tid == 0) sm.nnew = kept;
+            }
+        }
+        __syncthreads();
+        // w_q <- (w_q - sum_i o_iq b_i - sum_{p<q} L(q, p) w_p) / L(q, q)
+        const double *const L = sm.L;
+        for (int q0 = 0; q0 < na; q0 += 8) {
+            put_coefs(sm.cf, dimIter, q0, na, [&](int i, int q) { return sm.tot[i * na + q]; });
+            for (int k = tid; k < nc; k += DT) {
+                double x[8];
+#pragma unroll
+                for (int q = 0; q < 8; q++) x[q] = q0 + q < na ? W1[sm.act[q0 + q] * ld + k] : 0.0;
 #pragma unroll 4
                 for (int i = 0; i < dimIter; i++) {
-                    const double x = b.AB[cur][(size_t)i * n + k], y = b.B[cur][(size_t)i * n + k];
+                    const double v = Bl[i * ld + k];
 #pragma unroll
-                    for (int q = 0; q < RB; q++) {
-                        const double t = V[i * DAV_MAXD + col[q]];
-                        a[q] += t * x;
-                        c[q] += t * y;
+                    for (int q = 0; q < 4; q++) {
+                        const double2 f = sm.cf[i][q];
+                        x[2 * q] -= f.x * v;
+                        x[2 * q + 1] -= f.y * v;
                     }
                 }
+                if (pass > 0)
+                    for (int p = 0; p < q0; p++) {
+                        const double y = W1[sm.act[p] * ld + k];
 #pragma unroll
-                for (int q = 0; q < RB; q++)
-                    if (q < nr) {
-                        W0[(size_t)(r0 + q) * n + k] = a[q];
-                        W1[(size_t)(r0 + q) * n + k] = c[q];
+                        for (int q = 0; q < 8; q++)
+                            if (q0 + q < na) x[q] -= L[(q0 + q) * GL + p] * y;
+                    }
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    if (q0 + q < na) {
+                        if (pass > 0)
+#pragma unroll
+                            for (int p = 0; p < 8; p++)
+                                if (p < q) x[q] -= L[(q0 + q) * GL + q0 + p] * x[p];
+                        x[q] *= L[(q0 + q) * GL + q0 + q];
+                        W1[sm.act[q0 + q] * ld + k] = x[q];
                     }
             }
         }
-    }
-    __syncthreads();
-    block_dots(W1, W1, n, nroot, rd, rv);
-    for (int e = tid; e < nroot * n; e += DT) {
-        const int ir = e / n, k = e - ir * n;
-        const double t = sqrt(rv[ir]), ev = s.eigenVal[ir];
-        double q = W1[(size_t)ir * n + k], aq = W0[(size_t)ir * n + k];
-        if (fabs(t - 1.0) > 1.0e-10) {
-            q *= 1.0 / t;
-            aq *= 1.0 / t;
-        }
-        b.fileEV[(size_t)ir * (n + 1) + 1 + k] = q;
-        W1[(size_t)ir * n + k] = q;
-        W0[(size_t)ir * n + k] = aq - ev * q;
-    }
-    if (tid < nroot) b.fileEV[(size_t)tid * (n + 1)] = s.eigenVal[tid];
-    __syncthreads();
-    block_amaxs(W0, n, nroot, rd, ri, rv);
-    if (tid < nroot) {
-        cvd[tid] = fabs(rv[tid]) < s.maxError ? 1 : 0;
-        s.conv[tid] = cvd[tid];
-    }
-    __syncthreads();
-    int nNew = 0, nconv = 0;
-    for (int ir = 0; ir < nroot; ir++) nconv += cvd[ir];
-    for (int e = tid; e < nroot * n; e += DT) {
-        const int ir = e / n, k = e - ir * n;
-        if (cvd[ir]) continue;
-        double d = s.eigenVal[ir] - b.diag[k];
-        if (fabs(d) < 1.0e-4) d = (d < 0.0) ? -1.0e-4 : 1.0e-4;
-        W1[(size_t)ir * n + k] = W0[(size_t)ir * n + k] / d;
-    }
-    __syncthreads();
-    // SchmidtS (mod_davidson.f90:682-727): normalise, then project
-    block_dots(W1, W1, n, nroot, rd, rv);
-    for (int e = tid; e < nroot * n; e += DT) {
-        const int ir = e / n, k = e - ir * n;
-        if (!cvd[ir]) W1[(size_t)ir * n + k] *= 1.0 / sqrt(rv[ir]);
-    }
-    __syncthreads();
-    for (int ir = 0; ir < nroot; ir++) {
-        if (cvd[ir] || dimFree == 0) continue;
-        double *const w1 = W1 + (size_t)ir * n;
-        // projections on the basis: classical Gram-Schmidt applied twice
-        // (same result as the reference's sequential projections to
-        // rounding, with all overlaps of a pass computed at once)
-        const int nb = dimIter + nNew;
-        for (int pass = 0; pass < 2; pass++) {
-            for (int i = tid >> 5; i < nb; i += DT / 32) {
-                double v = warp_dot(b.B[cur] + (size_t)i * n, w1, n);
-                if ((tid & 31) == 0) ovl[i] = v;
-            }
-            __syncthreads();
-            for (int k = tid; k < n; k += DT) {
-                double x = w1[k];
-#pragma unroll 8
-                for (int i = 0; i < nb; i++) x += -ovl[i] * b.B[cur][(size_t)i * n + k];
-                w1[k] = x;
-            }
-            __syncthreads();
-        }
-        const double nrm = sqrt(block_dot(w1, w1, n, sh));
-        if (nrm < 1.0e-6) continue;
-        const int pos = dimIter + nNew;
-        for (int k = tid; k < n; k += DT) b.B[cur][(size_t)pos * n + k] = w1[k] * (1.0 / nrm);
         __syncthreads();
-        dimFree--;
-        nNew++;
-    }
-    if (tid == 0) {
-        s.cur = cur;
-        s.dimIter = dimIter;
-        s.dimFree = dimFree;
-        s.newpos = dimIter;
-        s.nNew = nNew;
-        if (nconv == nroot) {
-            s.done = 1;
-            s.converged = 1;
-        } else {
-            s.dim_exceed = 0;
-            if (dimFree == 0) {
-                s.dim_exceed = 1;
-                s.ndimIter = D - s.dimDel;
-                if (s.ndimIter < nroot) {
-                    s.ndimIter = nroot;
-                    s.ndimFree = D - s.ndimIter;
-                } else {
-                    s.ndimFree = s.dimDel;
+        if (pass == 1) {  // leave the dropped vectors out
+            nNew = sm.nnew;
+            if (nNew < na) {
+                if (tid == 0) {
+                    int m = 0;
+                    for (int q = 0; q < na; q++)
+                        if (L[q * GL + q] != 0.0) sm.act[m++] = sm.act[q];
                 }
+                na = nNew;
+                __syncthreads();
             }
         }
-        if (b.mailbox) {
-            b.mailbox[0] = s.done ? 0 : 1;
-            __threadfence_system();
+    }
+    // the new basis vectors, and their staged copies (zero beyond nNew) for a
+    // sigma launch whose size does not depend on nNew
+    for (int q = 0; q < nroot; q++)
+        for (int k = tid; k < nc; k += DT) {
+            const double x = q < nNew ? W1[sm.act[q] * ld + k] : 0.0;
+            if (q < nNew) b.B[cur][(size_t)(dimIter + q) * n + lo + k] = x;
+            b.W[(size_t)q * n + lo + k] = x;
+        }
+    if (t.rank == 0) {
+        if (tid < dimIter) {
+            s.valR[tid] = vR[tid];
+            s.lowestE[tid] = lw[tid];
+        }
+        if (tid < nroot) {
+            s.eigenVal[tid] = sm.ev[tid];
+            s.conv[tid] = sm.cvd[tid];
+            b.fileEV[(size_t)tid * (n + 1)] = sm.ev[tid];
+        }
+        if (tid == 0) {
+            dimFree -= nNew;
+            s.iterations = iterations;
+            s.cur = cur;
+            s.dimIter = dimIter;
+            s.dimFree = dimFree;
+            s.newpos = dimIter;
+            s.nNew = nNew;
+            s.nonsym_steps += general;
+            s.warn_imag += warn;
+            s.pending = 1;
+            if (nconv == nroot) {
+                s.done = 1;
+                s.converged = 1;
+                s.pending = 0;
+            } else {
+                s.dim_exceed = 0;
+                if (dimFree == 0) {
+                    s.dim_exceed = 1;
+                    s.ndimIter = D - s.dimDel;
+                    if (s.ndimIter < nroot) {
+                        s.ndimIter = nroot;
+                        s.ndimFree = D - s.ndimIter;
+                    } else {
+                        s.ndimFree = s.dimDel;
+                    }
+                }
+            }
+            if (b.mailbox) b.mailbox[0] = s.done ? 0 : 1;
         }
     }
-    // staged copies of the new basis vectors (zero beyond nNew) for a sigma
-    // launch whose size does not depend on nNew
-    if (b.W)
-        for (int q = 0; q < nroot; q++)
-            for (int k = tid; k < n; k += DT)
-                b.W[(size_t)q * n + k] = q < nNew ? b.B[cur][(size_t)(dimIter + q) * n + k] : 0.0;
+    t.leave();
 }
 
-// Ritz-matrix update with the new vectors (mod_davidson.f90:460-496); with
-// staged sigma vectors, AW[0..nNew) are first put in place in AB
-__global__ void __launch_bounds__(DT) k_dav_abar(DavState *st, DavBuffers b) {
-    DavState &s = *st;
+// Ritz-matrix update with the new vectors (mod_davidson.f90:460-496): the
+// staged sigma vectors AW[0..nNew) are put in place in AB and their products
+// with the basis formed, one CTA for the new vector blockIdx.x / ngroup and a
+// group of ABAR_G basis vectors: Abar(i, j) = b_i . Ab_j of the new column
+// j, and of the new row i for the older j (which hold no staged vector).
+// dimIter is that before the step's vectors; the next step counts them in.
+constexpr int ABAR_T = 256, ABAR_G = 4;
+__global__ void __launch_bounds__(ABAR_T) k_dav_abar(DavState *st, DavBuffers b, int ngroup) {
+    __shared__ double red[2 * ABAR_G][ABAR_T / 32];
+    const DavState &s = *st;
     if (s.done) return;
     const int n = s.dimA, D = s.D, dimIter = s.dimIter, nNew = s.nNew, cur = s.cur;
-    if (b.AW) {
-        for (int q = 0; q < nNew; q++)
-            for (int k = threadIdx.x; k < n; k += DT)
-                b.AB[cur][(size_t)(dimIter + q) * n + k] = b.AW[(size_t)q * n + k];
-        __syncthreads();
-    }
-    const double *B = b.B[cur], *AB = b.AB[cur];
-    // new rows (i >= dimIter, j < dimIter) then new columns (j >= dimIter)
-    const int nrow = nNew * dimIter, tot = nrow + nNew * (dimIter + nNew);
-    for (int e = threadIdx.x >> 5; e < tot; e += DT / 32) {
-        int i, j;
-        if (e < nrow) {
-            j = e / nNew;
-            i = dimIter + e % nNew;
-        } else {
-            j = dimIter + (e - nrow) / (dimIter + nNew);
-            i = (e - nrow) % (dimIter + nNew);
+    const int q = blockIdx.x / ngroup, g = blockIdx.x % ngroup;
+    const int i0 = g * ABAR_G, tot = dimIter + nNew;
+    if (q >= nNew || i0 >= tot) return;
+    const double *B = b.B[cur];
+    double *AB = b.AB[cur];
+    const double *aw = b.AW + (size_t)q * n, *bq = B + (size_t)(dimIter + q) * n;
+    double *ab = AB + (size_t)(dimIter + q) * n;
+    double col[ABAR_G], row[ABAR_G];
+#pragma unroll
+    for (int u = 0; u < ABAR_G; u++) col[u] = row[u] = 0.0;
+#pragma unroll 2
+    for (int k = threadIdx.x; k < n; k += ABAR_T) {
+        const double a = aw[k], x = bq[k];
+        if (g == 0) ab[k] = a;
+#pragma unroll
+        for (int u = 0; u < ABAR_G; u++) {
+            const int i = i0 + u;
+            if (i < tot) col[u] = fma(B[(size_t)i * n + k], a, col[u]);
+            if (i < dimIter) row[u] = fma(x, AB[(size_t)i * n + k], row[u]);
         }
-        double v = warp_dot(B + (size_t)i * n, AB + (size_t)j * n, n);
-        if ((threadIdx.x & 31) == 0) s.Abar[i + j * D] = v;
+    }
+    const int w = threadIdx.x >> 5;
+#pragma unroll
+    for (int u = 0; u < ABAR_G; u++) {
+        col[u] = warp_allsum(col[u]);
+        row[u] = warp_allsum(row[u]);
+        if ((threadIdx.x & 31) == 0) {
+            red[u][w] = col[u];
+            red[ABAR_G + u][w] = row[u];
+        }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        s.dimIter = dimIter + nNew;
-        s.iterations++;
+    if (threadIdx.x < 2 * ABAR_G) {
+        double v = 0.0;
+        for (int i = 0; i < ABAR_T / 32; i++) v += red[threadIdx.x][i];
+        const int i = i0 + (int)threadIdx.x % ABAR_G;
+        if (threadIdx.x < ABAR_G) {
+            if (i < tot) st->Abar[i + (dimIter + q) * D] = v;
+        } else if (i < dimIter) {
+            st->Abar[(dimIter + q) + i * D] = v;
+        }
     }
 }
 
@@ -1146,172 +1478,205 @@ __device__ void warp_dgesl(const double *a, int lda, int n, const int *ipvt, dou
     }
 }
 
-// R -= (<L|R> / ||L||) L, the reference's orthogonalR2L (which divides by
-// the norm, not its square)
-__device__ void block_orth(double *R, const double *L, int n, double *sh) {
-    // L.L and L.R in one pass and one reduction, each summed in
-    // block_dot's order (strided per-thread sums, shuffle-down, warp totals
-    // in warp order)
-    __shared__ double red[2][DT / 32];
-    double aa = 0.0, ab = 0.0;
-    for (int k = threadIdx.x; k < n; k += DT) {
-        const double l = L[k];
-        aa = fma(l, l, aa);
-        ab = fma(l, R[k], ab);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        aa += __shfl_down_sync(0xffffffffu, aa, o);
-        ab += __shfl_down_sync(0xffffffffu, ab, o);
-    }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        red[0][w] = aa;
-        red[1][w] = ab;
-    }
+// block sums of v[0..M) (and block maxima with MAX) of every thread, entry j
+// to out[j]; every thread calls it, the caller's barrier publishes out
+template <int M, bool MAX = false>
+__device__ void block_reduce(const double (&v)[M], double (*red)[DT / 32], double *out) {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    double x[M];
+#pragma unroll
+    for (int j = 0; j < M; j++) x[j] = MAX ? warp_allmax(v[j]) : warp_allsum(v[j]);
+    if (lane == 0)
+#pragma unroll
+        for (int j = 0; j < M; j++) red[j][w] = x[j];
     __syncthreads();
-    if (threadIdx.x < 2) {
-        double t = 0.0;
-        for (int i = 0; i < DT / 32; i++) t += red[threadIdx.x][i];
-        sh[threadIdx.x] = t;
+    if (threadIdx.x < M) {
+        double t = MAX ? -1.0 : 0.0;
+        for (int i = 0; i < DT / 32; i++) t = MAX ? fmax(t, red[threadIdx.x][i]) : t + red[threadIdx.x][i];
+        out[threadIdx.x] = t;
     }
-    __syncthreads();
-    double nrm = sqrt(sh[0]);
-    double dot = sh[1];
-    __syncthreads();
-    double f = -dot / nrm;
-    for (int k = threadIdx.x; k < n; k += DT) R[k] += f * L[k];
     __syncthreads();
 }
 
-__device__ void diis_extrapolate(DiisState &s, const DiisBuffers &b, double *vec, double *sh, int *shi, double *Bm,
-                                 double *coef, double *aug, double *rhs, int *ipvt);
-
-// R *= 1 / <R|V> (the left vector's normalisation to the right one,
-// calEigenCISDoo.f90:99-104: a dscal by the reciprocal)
-__device__ void block_unit_dot(double *R, const double *V, int n, double *sh) {
-    const double d = 1.0 / block_dot(R, V, n, sh);
-    __syncthreads();
-    for (int k = threadIdx.x; k < n; k += DT) R[k] *= d;
-    __syncthreads();
-}
-
-// one step of the device-driven solver for root blockIdx.x (see solvers.cuh)
+// One step of the device-driven solver (see solvers.cuh) for the root of this
+// cluster.  Short R1 vectors are latency-bound (one CTA; up to three
+// exchanges a step), the (R1, R2) vectors of the grCPS(D) programs
+// bandwidth-bound: 2 x diis_dim stored vectors are read a step, by 16 SMs
+// (27 k elements: 165 us a step on one).
+//   1. R1 = pr / den and the sums of orthogonalR2L (R -= (<L|R> / ||L||) L:
+//      the reference divides by the norm, not its square) or <R1|nrmv>;
+//   2. that correction, the DIIS error vector and its overlaps;
+//   3. the bordered system (every CTA for itself), the extrapolated vector,
+//      its residual and the sums of the second correction;
+//   4. the second correction.
 __global__ void __launch_bounds__(DT) k_solver_step(SolverArgs a) {
-    __shared__ double sh[DT / 32 + 1];
-    __shared__ int shi[DT / 32 + 1];
-    __shared__ double Bm[DIIS_MAXDIM * DIIS_MAXDIM];
+    __shared__ double red[DIIS_MAXDIM][DT / 32], ex[2][DIIS_MAXDIM], tot[DIIS_MAXDIM];
+    __shared__ double Bm[DIIS_MAXDIM * DIIS_MAXDIM], row[DIIS_MAXDIM];
     __shared__ double coef[DIIS_MAXDIM + 1];
     __shared__ double aug[(DIIS_MAXDIM + 1) * (DIIS_MAXDIM + 1)], rhs[DIIS_MAXDIM + 1];
     __shared__ int ipvt[DIIS_MAXDIM + 1];
-    const int r = blockIdx.x, tid = threadIdx.x, len = a.len;
+    const int len = a.len, tid = threadIdx.x;
+    Team t(len);
+    const int r = blockIdx.x / t.size;
     SolverState &ss = a.ss[r];
-    if (!ss.active) return;
-    const int iter = ss.iter + 1;
-    double *pr = a.pr + (size_t)r * len, *R1 = a.R1 + (size_t)r * len;
-    const double *cc = a.cc + (size_t)r * len, *S = a.S + (size_t)r * len;
-    const double *L = a.L ? a.L + (size_t)r * len : nullptr;
-    if (iter > 1) {  // pr = cc; pr += (-w0) R1; pr += sigma  (the reference's updates, in order)
-        if (a.w0) {
-            const double mw0 = -a.w0[r];
-            for (int k = tid; k < len; k += DT) pr[k] = fma(mw0, R1[k], cc[k]) + S[k];
-        } else {
-            for (int k = tid; k < len; k += DT) pr[k] = cc[k] + S[k];
-        }
-        __syncthreads();
-    }
-    if (iter > 1 || !a.keep_first)
-        for (int k = tid; k < len; k += DT) R1[k] = pr[k] / a.den[k];
-    __syncthreads();
-    const double *NV = a.nrmv ? a.nrmv + (size_t)r * len : nullptr;
     DiisState &ds = a.ds[r];
-    DiisBuffers b;
-    b.prev = a.db.prev + (size_t)r * a.sprev;
-    b.err = a.db.err + (size_t)r * a.serr;
-    b.amp = a.db.amp + (size_t)r * a.serr;
-    if (L) block_orth(R1, L, len, sh);
-    if (NV) block_unit_dot(R1, NV, len, sh);
+    const bool active = ss.active;
+    const int iter = ss.iter + 1, maxdim = ds.maxdim, id = ds.idimr - 1, nd = ds.ndimr;
+    for (int e = tid; e < DIIS_MAXDIM * DIIS_MAXDIM; e += DT) Bm[e] = ds.Bm[e];
+    t.sync();  // every CTA has read the state
+    if (!active) return;
+    const size_t o = (size_t)r * len;
+    double *pr = a.pr + o, *R1 = a.R1 + o;
+    const double *cc = a.cc + o, *S = a.S + o;
+    const double *L = a.L ? a.L + o : nullptr, *NV = a.nrmv ? a.nrmv + o : nullptr;
+    double *prev = a.db.prev + (size_t)r * a.sprev, *err = a.db.err + (size_t)r * a.serr;
+    double *amp = a.db.amp + (size_t)r * a.serr;
+    const double *U = L ? L : NV;  // the vector of the two corrections
+    double ll = 0.0;               // ||L||
+    // ---- 1
+    double s2[2] = {0.0, 0.0};
+    const double mw0 = a.w0 ? -a.w0[r] : 0.0;
+    for (int k = t.lo + tid; k < t.hi; k += DT) {
+        double x;
+        if (iter > 1) {  // pr = cc; pr += (-w0) R1; pr += sigma  (the reference's updates, in order)
+            x = (a.w0 ? fma(mw0, R1[k], cc[k]) : cc[k]) + S[k];
+            pr[k] = x;
+        } else {
+            x = pr[k];
+        }
+        double v = (iter > 1 || !a.keep_first) ? x / a.den[k] : R1[k];
+        R1[k] = v;
+        if (U) {
+            const double u = U[k];
+            s2[0] = fma(u, u, s2[0]);
+            s2[1] = fma(u, v, s2[1]);
+        }
+    }
+    double f = 0.0, g = 1.0;  // the correction R1 = g (R1 + f U)
+    if (U) {
+        double *part = t.next(ex[0], DIIS_MAXDIM);
+        block_reduce(s2, red, part);
+        t.sync();
+        const double uu = t.sum(part, 0), ur = t.sum(part, 1);
+        if (L) {
+            ll = sqrt(uu);
+            f = -ur / ll;
+        } else {
+            g = 1.0 / ur;
+        }
+    }
+    // ---- 2
     if (iter == 1) {
-        for (int k = tid; k < len; k += DT) b.prev[k] = R1[k];
-        if (tid == 0) {
-            ds.idimr = 1;
-            ds.ndimr = 1;
-            ds.res = 1.0;
+        double s1[2] = {0.0, 0.0};
+        for (int k = t.lo + tid; k < t.hi; k += DT) {
+            double v = R1[k];
+            if (L) v += f * L[k];
+            v *= g;
+            R1[k] = v;
+            prev[k] = v;
+            if (U) s1[1] = fma(U[k], v, s1[1]);
+        }
+        if (U) {
+            double *part = t.next(ex[0], DIIS_MAXDIM);
+            block_reduce(s1, red, part);
+            t.sync();
+            const double ur = t.sum(part, 1);
+            if (L) f = -ur / ll;
+            else g = 1.0 / ur;
         }
     } else {
-        diis_extrapolate(ds, b, R1, sh, shi, Bm, coef, aug, rhs, ipvt);
+        double dt[DIIS_MAXDIM];
+#pragma unroll
+        for (int j = 0; j < DIIS_MAXDIM; j++) dt[j] = 0.0;
+        for (int k = t.lo + tid; k < t.hi; k += DT) {
+            double v = R1[k];
+            if (L) v += f * L[k];
+            v *= g;
+            const double p = prev[k], e = v - p;
+            amp[(size_t)id * len + k] = p;
+            err[(size_t)id * len + k] = e;
+#pragma unroll
+            for (int j = 0; j < DIIS_MAXDIM; j++)
+                if (j < nd) dt[j] = fma(e, j == id ? e : err[(size_t)j * len + k], dt[j]);
+        }
+        double *part = t.next(ex[0], DIIS_MAXDIM);
+        block_reduce(dt, red, part);
+        t.sync();
+        // only the row of the error vector stored now changes; the others
+        // are kept in the state from earlier steps
+        if (tid < nd) {
+            const double x = t.sum(part, tid);
+            row[tid] = x;
+            Bm[id + tid * DIIS_MAXDIM] = x;
+            Bm[tid + id * DIIS_MAXDIM] = x;
+        }
+        __syncthreads();
+        // ---- 3
+        if (tid < 32) {  // dodiis (src/libsrint/dodiis.f): bordered system with -1e-4
+            const int n1 = nd + 1;
+            for (int e = tid; e < n1 * n1; e += 32) {
+                const int i = e % n1, j = e / n1;
+                aug[e] = (i == 0 && j == 0) ? 0.0
+                         : (i == 0 || j == 0) ? -1.0e-4
+                                              : Bm[(i - 1) + (j - 1) * DIIS_MAXDIM];
+            }
+            if (tid < n1) rhs[tid] = (tid == 0) ? -1.0e-4 : 0.0;
+            __syncwarp();
+            warp_dgefa(aug, n1, n1, ipvt);
+            warp_dgesl(aug, n1, n1, ipvt, rhs);
+            if (tid < nd) coef[tid] = rhs[tid + 1];
+        }
+        __syncthreads();
+        double s1[1] = {0.0}, big[1] = {-1.0};
+        for (int k = t.lo + tid; k < t.hi; k += DT) {
+            double v = 0.0, p = 0.0;
+#pragma unroll 4
+            for (int i = 0; i < nd; i++) {
+                v += coef[i] * err[(size_t)i * len + k];
+                p += coef[i] * amp[(size_t)i * len + k];
+            }
+            if (fabs(v) > big[0]) big[0] = fabs(v);
+            v += p;
+            prev[k] = v;
+            R1[k] = v;
+            if (U) s1[0] = fma(U[k], v, s1[0]);
+        }
+        part = t.next(ex[0], DIIS_MAXDIM);
+        block_reduce<1, true>(big, red, part);
+        block_reduce(s1, red, part + 1);
+        t.sync();
+        const double res = fmax(t.amax(part, 0), 0.0), ur = t.sum(part, 1);
+        if (tid == 0) tot[0] = res;
+        f = 0.0;
+        g = 1.0;
+        if (L) f = -ur / ll;
+        else if (NV) g = 1.0 / ur;
     }
-    __syncthreads();
-    if (L) block_orth(R1, L, len, sh);
-    if (NV) block_unit_dot(R1, NV, len, sh);
-    if (tid == 0) {
-        const double res = ds.res;
-        ss.iter = iter;
-        ss.res = res;
-        if ((iter > 1 && fabs(res) < a.tol) || iter > a.cyc) ss.active = 0;
-        a.mailbox[r] = ss.active;
-        __threadfence_system();
-    }
-}
-
-__device__ void diis_extrapolate(DiisState &s, const DiisBuffers &b, double *vec, double *sh, int *shi, double *Bm,
-                                 double *coef, double *aug, double *rhs, int *ipvt) {
-    const int len = s.len, maxdim = s.maxdim, tid = threadIdx.x;
-    const int id = s.idimr - 1;
-    for (int k = tid; k < len; k += DT) {
-        double p = b.prev[k];
-        b.amp[(size_t)id * len + k] = p;
-        double e = vec[k] - p;
-        vec[k] = e;
-        b.err[(size_t)id * len + k] = e;
-    }
-    __syncthreads();
-    const int nd = s.ndimr;
-    // only the row of the error vector stored now changes; the others are
-    // kept in the state from earlier steps
-    for (int j = tid >> 5; j < nd; j += DT / 32) {
-        double x = warp_dot(b.err + (size_t)id * len, b.err + (size_t)j * len, len);
-        if ((tid & 31) == 0) {
-            s.Bm[id + j * DIIS_MAXDIM] = x;
-            s.Bm[j + id * DIIS_MAXDIM] = x;
+    // ---- 4
+    if (U)
+        for (int k = t.lo + tid; k < t.hi; k += DT) {
+            double v = R1[k];
+            if (L) v += f * L[k];
+            R1[k] = v * g;
+        }
+    if (t.rank == 0) {
+        if (iter > 1 && tid < nd) {
+            ds.Bm[id + tid * DIIS_MAXDIM] = row[tid];
+            ds.Bm[tid + id * DIIS_MAXDIM] = row[tid];
+        }
+        if (tid == 0) {
+            const double res = iter > 1 ? tot[0] : 1.0;
+            ds.res = res;
+            ds.ndimr = iter > 1 ? ((nd + 1 < maxdim) ? nd + 1 : maxdim) : 1;
+            ds.idimr = iter > 1 ? (id + 2 > maxdim ? 1 : id + 2) : 1;
+            ss.iter = iter;
+            ss.res = res;
+            const int go = !((iter > 1 && fabs(res) < a.tol) || iter > a.cyc);
+            ss.active = go;
+            a.mailbox[r] = go;
         }
     }
-    __syncthreads();
-    for (int e = tid; e < DIIS_MAXDIM * DIIS_MAXDIM; e += DT) Bm[e] = s.Bm[e];
-    __syncthreads();
-    if (tid < 32) {  // dodiis (src/libsrint/dodiis.f): bordered system with -1e-4
-        const int n1 = nd + 1;
-        for (int e = tid; e < n1 * n1; e += 32) {
-            const int i = e % n1, j = e / n1;
-            aug[e] = (i == 0 && j == 0) ? 0.0
-                     : (i == 0 || j == 0) ? -1.0e-4
-                                          : Bm[(i - 1) + (j - 1) * DIIS_MAXDIM];
-        }
-        if (tid < n1) rhs[tid] = (tid == 0) ? -1.0e-4 : 0.0;
-        __syncwarp();
-        warp_dgefa(aug, n1, n1, ipvt);
-        warp_dgesl(aug, n1, n1, ipvt, rhs);
-        if (tid < nd) coef[tid] = rhs[tid + 1];
-    }
-    __syncthreads();
-    for (int k = tid; k < len; k += DT) {
-        double v = 0.0;
-        for (int i = 0; i < nd; i++) v += coef[i] * b.err[(size_t)i * len + k];
-        vec[k] = v;
-    }
-    __syncthreads();
-    double res = block_amax(vec, len, sh, shi);
-    for (int k = tid; k < len; k += DT) {
-        double v = vec[k];
-        for (int i = 0; i < nd; i++) v += coef[i] * b.amp[(size_t)i * len + k];
-        vec[k] = v;
-        b.prev[k] = v;
-    }
-    if (tid == 0) {
-        s.res = res;
-        s.ndimr = (nd + 1 < maxdim) ? nd + 1 : maxdim;
-        s.idimr = s.idimr + 1;
-        if (s.idimr > maxdim) s.idimr = 1;
-    }
+    t.leave();
 }
 
 // the general eigen-solve of the Davidson step on one given matrix
@@ -1326,7 +1691,7 @@ __global__ void __launch_bounds__(32) k_geev_probe(const double *A, int n, doubl
         wr[threadIdx.x] = r[threadIdx.x];
         wi[threadIdx.x] = im[threadIdx.x];
     }
-    for (int e = threadIdx.x; e < n * n; e += 32) V[e] = Z[(e / n) * DAV_MAXD + e % n];
+    for (int e = threadIdx.x; e < n * n; e += 32) V[e] = Z[(e / n) * GL + e % n];
     if (threadIdx.x == 0) *sweeps = sw;
 }
 
@@ -1344,18 +1709,27 @@ int dav_init_launch(DavState *st, const DavBuffers &b) {
     count_launch();
     return cuda_check(cudaGetLastError(), "k_dav_init");
 }
-int dav_step_launch(DavState *st, const DavBuffers &b) {
+int dav_step_launch(DavState *st, const DavBuffers &b, i64 n, int nroot, int D) {
+    constexpr size_t base = (sizeof(DavShared) + 15) / 16 * 16, most = base + sizeof(double) * DAV_LOCAL;
+    static_assert(most + 1024 <= 227 * 1024, "shared memory of a Davidson step");
+    static std::atomic<bool> attr{false};
+    CPSD_TRY(team_attrs(k_dav_step, most, attr));
     cudaEvent_t end;
     CPSD_TRY(timing_begin(0.0, 0, 0, 0, 30, &end));
-    k_dav_step<<<1, DT, 0, stream()>>>(st, b);
+    const int size = team_size(n, DAV_PER);
+    const int nc = (int)(((n + size - 1) / size + 31) & ~(i64)31);
+    const i64 need = (i64)2 * (D + nroot) * dav_ld(nc);
+    const int local = need <= DAV_LOCAL;
+    CPSD_TRY(launch_team(k_dav_step, 1, size, base + (local ? sizeof(double) * (size_t)need : 0), "k_dav_step", st, b,
+                         local));
     count_launch();
-    CPSD_TRY(cuda_check(cudaGetLastError(), "k_dav_step"));
     return timing_end(end);
 }
-int dav_abar_launch(DavState *st, const DavBuffers &b) {
+int dav_abar_launch(DavState *st, const DavBuffers &b, int nroot, int D) {
     cudaEvent_t end;
     CPSD_TRY(timing_begin(0.0, 0, 0, 0, 31, &end));
-    k_dav_abar<<<1, DT, 0, stream()>>>(st, b);
+    const int ngroup = (D + ABAR_G - 1) / ABAR_G;
+    k_dav_abar<<<nroot * ngroup, ABAR_T, 0, stream()>>>(st, b, ngroup);
     count_launch();
     CPSD_TRY(cuda_check(cudaGetLastError(), "k_dav_abar"));
     return timing_end(end);
@@ -1368,11 +1742,12 @@ int dav_final_launch(DavState *st, const DavBuffers &b) {
 }
 int solver_step_launch(const SolverArgs &a) {
     if (a.nb <= 0) return CPSD_OK;
+    static std::atomic<bool> attr{false};
+    CPSD_TRY(team_attrs(k_solver_step, 0, attr));
     cudaEvent_t end;
     CPSD_TRY(timing_begin(0.0, a.nb, 0, 0, 32, &end));
-    k_solver_step<<<a.nb, DT, 0, stream()>>>(a);
+    CPSD_TRY(launch_team(k_solver_step, a.nb, team_size(a.len, DT), 0, "k_solver_step", a));
     count_launch();
-    CPSD_TRY(cuda_check(cudaGetLastError(), "k_solver_step"));
     return timing_end(end);
 }
 

@@ -15,17 +15,14 @@ struct DavState {
     // steps that took the general (non-symmetric) eigen-solve, Ritz values
     // with an imaginary part above 1e-10 (the reference's warning,
     // mod_davidson.f90:193-196), QR iteration failure
-    int nonsym_steps, warn_imag, eig_fail, pad;
+    int nonsym_steps, warn_imag, eig_fail;
+    int pending;  // the last step's nNew vectors are not yet counted in dimIter
     double maxError, max_resid;
     int conv[DAV_MAXD];
     int lowestE[DAV_MAXD];
     double eigenVal[DAV_MAXD];
     double valR[DAV_MAXD];
     double Abar[DAV_MAXD * DAV_MAXD];
-    double vecR[DAV_MAXD * DAV_MAXD];
-    double vecNeed[DAV_MAXD * DAV_MAXD];
-    double oldE[DAV_MAXD * DAV_MAXD];
-    double newE[DAV_MAXD * DAV_MAXD];
 };
 
 struct DavBuffers {
@@ -36,13 +33,13 @@ struct DavBuffers {
     // device-driven loop: the step stages its new vectors in W (nroot x dimA,
     // zero beyond nNew), the sigma of W goes to AW and the Ritz update moves
     // it in place; mailbox[0] (mapped host memory) = 1 while iterating
-    double *W = nullptr, *AW = nullptr;
+    double *W = nullptr, *AW = nullptr;  // never null in the step and update launches
     int *mailbox = nullptr;
 };
 
 int dav_init_launch(DavState *st, const DavBuffers &b);      // Abar of the guesses
-int dav_step_launch(DavState *st, const DavBuffers &b);
-int dav_abar_launch(DavState *st, const DavBuffers &b);
+int dav_step_launch(DavState *st, const DavBuffers &b, i64 n, int nroot, int D);
+int dav_abar_launch(DavState *st, const DavBuffers &b, int nroot, int D);
 int dav_final_launch(DavState *st, const DavBuffers &b);     // eigen test residual
 // the Davidson step's general eigen-solve on one row-major n x n device
 // matrix: eigenvalues wr / wi, eigenvectors V (row-major, dgeev's columns),
@@ -61,8 +58,8 @@ struct DiisBuffers {
 // Device-driven solver steps for nb independent roots: the EE solver
 // (solver.f90:4-66), without L and w0 the ground T1^(2) DIIS loop
 // (run2.f90) and the grCPS(D) (T1, T2) loop, with nrmv the CIS(D-infinity)
-// left-vector loop (src/EE-grCPSd.SF/calEigenCISDoo.f90:94-140).  One CTA
-// per root and step does
+// left-vector loop (src/EE-grCPSd.SF/calEigenCISDoo.f90:94-140).  One
+// cluster of CTAs per root and step does
 //   pr = cc - w0 R1 + S      (S = the sigma of the previous step's R1; from step 2)
 //   R1 = pr / den (den = ei - ea, or ei + ej - ea - eb on the doubles; kept
 //   as given at step 1 with keep_first);  orthogonalR2L or the <R1|nrmv> = 1
