@@ -8,6 +8,7 @@
 #include "drivers.hpp"
 #include "narrow.cuh"
 #include "ozaki.cuh"
+#include "pairblk.cuh"
 #include "rowdot.cuh"
 #include "shortk.cuh"
 #include "solvers.cuh"
@@ -79,6 +80,18 @@ static void trace_contraction(const ContractPlan *p, const char *t1, const char 
             out * (double)(nb > 1 ? nb : 1));
 }
 
+// digit tensor-core path for large contractions whose dense regrouping uses
+// at least a quarter of the padded tiles and has K of at least 256
+// (min_gflop = 0 routes every contraction that regroups); nullptr: not taken
+static int digit_route(const ContractPlan *p, const OzPlan **oz) {
+    *oz = nullptr;
+    if (ctx().oz_digits > 0 && !p->empty && p->flops >= ctx().oz_min_flops) {
+        CPSD_TRY(plan_ozaki(p, ctx().oz_digits, oz));
+        if (*oz && ctx().oz_min_flops > 0 && ((*oz)->pad_eff < 0.25 || (*oz)->kmin < 256)) *oz = nullptr;
+    }
+    return CPSD_OK;
+}
+
 int engine(const Ten &v1, const char *t1, const Ten &v2, const char *t2, Ten &v3, const char *t3, double f1,
            double f2, i64 nb) {
     CPSD_TRY(need_init());
@@ -92,14 +105,8 @@ int engine(const Ten &v1, const char *t1, const Ten &v2, const char *t2, Ten &v3
     }
     const ContractPlan *p;
     CPSD_TRY(plan_contract(v1.d, t1, v2.d, t2, v3.d, t3, b, &p));
-    // digit tensor-core path for large contractions whose dense regrouping
-    // uses at least a quarter of the padded tiles and has K of at least 256
-    // (min_gflop = 0 routes every contraction that regroups)
     const OzPlan *oz = nullptr;
-    if (ctx().oz_digits > 0 && !p->empty && p->flops >= ctx().oz_min_flops) {
-        CPSD_TRY(plan_ozaki(p, ctx().oz_digits, &oz));
-        if (oz && ctx().oz_min_flops > 0 && (oz->pad_eff < 0.25 || oz->kmin < 256)) oz = nullptr;
-    }
+    CPSD_TRY(digit_route(p, &oz));
     i64 l3 = v3.len();
     if (f2 != 1.0) {
         if (nb <= 1 || b.strideC == l3) CPSD_TRY(launch_scale(v3.arr, l3 * (nb > 1 ? nb : 1), f2));
@@ -858,6 +865,39 @@ int vjp444(const Ten &v1, const Ten &v2, const Ten &Y, Ten &G, int which, double
     return launch_pairmap(pm, E.arr, G.arr, 1.0, 1.0);
 }
 
+namespace {
+// A packed (vv|vo) list times singles by the kernels that read it packed,
+// unless the mixed mode would send the expanded contraction to the digit
+// path (*done stays false: the caller takes the general path).  No expanded
+// copy is made or kept.
+int packed_singles(const Ten &V, const char *tv, const Ten &r, const char *tr, Ten &out, const char *to, i64 nb,
+                   int (*run)(const Ten &, const Ten &, Ten &, double, i64, bool *), double f, bool *done) {
+    CPSD_TRY(need_init());
+    if (V.d.iop[0] != 0) return CPSD_OK;
+    OpScope op;
+    Desc full = V.d;
+    full.iop[0] = 1;
+    Batch b;
+    b.nb = nb;
+    if (nb > 1) {
+        b.strideB = r.bs;
+        b.strideC = out.bs ? out.bs : out.len();
+    }
+    const ContractPlan *p;
+    CPSD_TRY(plan_contract(full, tv, r.d, tr, out.d, to, b, &p));
+    if (p->empty) return CPSD_OK;
+    const OzPlan *oz = nullptr;
+    CPSD_TRY(digit_route(p, &oz));
+    if (oz) return CPSD_OK;
+    CPSD_TRY(run(V, r, out, f, nb, done));
+    if (*done) {
+        trace_contraction(p, tv, tr, to, nb, "packed pair");
+        ctx().flops += p->flops;
+    }
+    return CPSD_OK;
+}
+}  // namespace
+
 // ------------------------------------------------ lib_cc kernels (spin-free)
 int k_c1_r1iabj(Ten &c1, const Ten &r1, const Ten &V, double f, i64 nb) {
     return w422(V, r1, c1, f, "fnai", "fn", "ai", nb);
@@ -997,6 +1037,9 @@ int k_Fmi_r1ijka(Ten &F, const Ten &r1, const Ten &V, double f, i64 nb) {
     return w422(V, r1, F, f, "mnie", "en", "mi", nb);
 }
 int k_Fae_r1abci(Ten &F, const Ten &r1, const Ten &V, double f, i64 nb) {
+    bool done = false;
+    CPSD_TRY(packed_singles(V, "efam", r1, "fm+-", F, "ae+-", nb, pairblk_fae, f, &done));
+    if (done) return CPSD_OK;
     return w422(V, r1, F, f, "efam", "fm", "ae", nb);
 }
 int k_Wkbij_r2ijka(Ten &W, const Ten &r2, const Ten &V, double f, i64 nb) {
@@ -1024,6 +1067,9 @@ int k_Wmbej_r2abij(Ten &W, const Ten &r2, const Ten &V, double f, i64 nb) {
     return w444(V, r2, W, 0.5 * f, "fenm", "bfjn", "embj", 0, nb);
 }
 int k_Wmbej_r1abci(Ten &W, const Ten &r1, const Ten &V, double f, i64 nb) {
+    bool done = false;
+    CPSD_TRY(packed_singles(V, "febm", r1, "fj..", W, "embj", nb, pairblk_wmbej, f, &done));
+    if (done) return CPSD_OK;
     return w424(V, r1, W, f, "febm", "fj", "embj", 0, nb);
 }
 int k_Wmbej_r1ijka(Ten &W, const Ten &r1, const Ten &V, double f, i64 nb) {

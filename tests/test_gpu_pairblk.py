@@ -1,0 +1,58 @@
+"""The kernels that read the packed (vv|vo) list (Wmbej_r1abci, Fae_r1abci)
+against the oracle where they can go wrong: one to three chunks of 96 rows
+with remainders, row tiles of 8 and strips of 8 at and beside their edges,
+more than eight columns, singles of another irrep than 1, irreps without
+occupied orbitals, every tile-count instance.
+
+Operands are standard normal, so an output is a sum of at most 2 x 212 terms of
+size 1: its FP64 rounding is below 424 eps sqrt(424) = 2e-12, in either order.
+"""
+import numpy as np
+import pytest
+
+import kernel_specs as ks
+import oracle_ffi as of
+from cpsd_b200 import api, synth
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("name", ["Wmbej_r1abci", "Fae_r1abci"])
+@pytest.mark.parametrize("nmo,nocc,nirrep,symr", [
+    (110, (3, 1), 1, 1),   # v = 216: three chunks
+    (52, (5, 3), 1, 1),    # v = 96: one full chunk
+    (53, (5, 4), 1, 1),    # v = 97, nine columns
+    (20, (4, 2), 1, 1),    # v = 34: the 8-tile instance
+    (13, (2, 1), 1, 1),    # v = 23: the 4-tile instance
+    (90, (7, 5), 2, 2),    # irreps of 84, singles of irrep 2
+    (37, (5, 3), 4, 3),
+    (35, (3, 1), 8, 1),    # irreps without occupied orbitals
+    (35, (9, 7), 8, 6),
+])
+def test_packed_pair_matches_oracle(name, nmo, nocc, nirrep, symr):
+    rng = np.random.default_rng(nmo)
+    s = synth.System(nmo=nmo, nocc_a=nocc[0], nocc_b=nocc[1], nirrep=nirrep, seed=2, naux=nirrep, skip_abcd=True,
+                     host_ints=False)
+    api.use_torch_stream()
+    api.init(s.nirrep, s.dirprd)
+    of.set_symmetry(s.nirrep, s.dirprd)
+    lo, la, lb, _ = ks.KERNELS[name]
+    ops = []
+    for layout, sym in ((lo, symr), (la, symr), (lb, 1)):
+        pops, iops = ks.pops_of(layout, s.popo, s.popv)
+        n = s.sym.idsymsoc(sym, pops[0], pops[1], iops[0], pops[2], pops[3], iops[1])
+        ops.append((pops, iops, sym, rng.standard_normal(n)))
+    ref = ops[0][3].copy()
+    args = [of.opt(p, i, y, x) for p, i, y, x in ops]
+    args[0] = of.opt(*ops[0][:3], ref)
+    assert of.call_kernel(name, *args, 0.7) == 0
+    dev = [torch.from_numpy(x).cuda() for _, _, _, x in ops]
+    api.contract_timing(True)
+    try:
+        api.kernel(name, *[api.opt(p, i, y, t) for (p, i, y, _), t in zip(ops, dev)], 0.7)
+        _, _, kinds, _ = api.contract_records()
+    finally:
+        api.contract_timing(False)
+    assert 23 in kinds and 40 not in kinds, "the list was expanded"
+    assert float(np.max(np.abs(dev[0].cpu().numpy() - ref))) < 2e-12 * (1 + np.max(np.abs(ref)) / 50)
