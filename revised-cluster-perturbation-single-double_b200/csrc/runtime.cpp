@@ -72,16 +72,12 @@ i64 Desc::block_base(i64 R) const {
     return b;
 }
 
+// the descriptor's bytes (formatting the numbers took longer than a launch)
 std::string Desc::key() const {
-    std::string s;
-    char buf[32];
-    for (int k = 0; k < 4; k++)
-        for (int i = 0; i < 8; i++) {
-            snprintf(buf, sizeof buf, "%lld,", (long long)pop[k][i]);
-            s += buf;
-        }
-    snprintf(buf, sizeof buf, "|%lld%lld|%lld", (long long)iop[0], (long long)iop[1], (long long)sym);
-    return s + buf;
+    std::string s(reinterpret_cast<const char *>(pop), sizeof pop);
+    s.append(reinterpret_cast<const char *>(iop), sizeof iop);
+    s.append(reinterpret_cast<const char *>(&sym), sizeof sym);
+    return s;
 }
 
 Desc make_desc(const i64 *p0, const i64 *p1, const i64 *p2, const i64 *p3, i64 iop0, i64 iop1, i64 sym) {
