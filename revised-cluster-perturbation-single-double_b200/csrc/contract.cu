@@ -5,10 +5,13 @@
 // task (the irrep assignments of the contracted indices), gathering A / B
 // tiles through the planner's stride tables (packed pairs are composite
 // indices) into padded shared memory and multiplying them on the FP64
-// tensor pipe with mma.sync.m8n8k4.f64 (tcgen05 has no FP64 kind).  The
-// next K stage is fetched into registers while the current one is
-// multiplied.  Split-K tiles write partial sums that k_splitk_reduce adds
-// in a fixed order, so results are deterministic.
+// tensor pipe with mma.sync.m8n8k4.f64 (tcgen05 has no FP64 kind).  K stages
+// of 16 are copied with cp.async into a ring, two or three stages ahead of
+// the one that is multiplied, one barrier a stage; staging them in registers
+// one stage ahead was slower in every shape (128x32 on the C1 nmo-71 ladder:
+// 517 us against 256).  Split-K tiles write
+// partial sums that k_splitk_reduce adds in a fixed order, so results are
+// deterministic.
 #include <atomic>
 #include <array>
 #include <vector>
@@ -22,6 +25,11 @@ namespace cpsd {
 
 namespace {
 constexpr int NT = 256, BK = 16, PAD = 4;
+// K stages in the ring: four, or three where that lets a third CTA onto the SM
+// (four warps with 32 x 32 of the tile each).  The 128x16 tile streams its
+// first operand and is better off with the deeper ring (19 columns in 8 irreps
+// of 9100 pairs: 1.33 ms with four stages, 1.63 with three).
+constexpr int ring(int warps, int bn) { return warps == 4 && bn > 16 ? 3 : 4; }
 
 __device__ __forceinline__ i64 decode1(i64 x, int n, const i64 *ext, const i64 *st) {
     // the last unit takes the remaining quotient whole (x < its extent), so
@@ -42,132 +50,161 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 
-template <int BM, int BN>
+template <int BM, int BN, int WARPS>
 constexpr int smem_bytes() {
-    return (int)sizeof(double) * 2 * BK * ((BM + PAD) + (BN + PAD));
+    return (int)sizeof(double) * ring(WARPS, BN) * BK * ((BM + PAD) + (BN + PAD));
+}
+
+// 8-byte asynchronous copy, or zero fill without reading the source
+__device__ __forceinline__ void stage_cp(double *dst, const double *src, bool read) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(read ? 8 : 0)
+                 : "memory");
+}
+// a table entry by the threads of a CTA, one word each
+template <class T>
+__device__ __forceinline__ void copy_entry(T *dst, const T *src) {
+    static_assert(sizeof(T) % 8 == 0 && sizeof(T) / 8 <= 128, "words of a table entry");
+    if (threadIdx.x < sizeof(T) / 8)
+        reinterpret_cast<long long *>(dst)[threadIdx.x] = reinterpret_cast<const long long *>(src)[threadIdx.x];
 }
 
 template <int BM, int BN, int WM, int WN>
-__global__ void __launch_bounds__(NT, 2) k_contract(const double *__restrict__ A, const double *__restrict__ B,
+__global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract(const double *__restrict__ A, const double *__restrict__ B,
                                                     double *__restrict__ C, const TaskDev *__restrict__ tasks,
                                                     const SegDev *__restrict__ segs, const TileDev *__restrict__ tiles,
                                                     double alpha, double *__restrict__ partial) {
-    static_assert(WM * WN == NT / 32, "8 warps");
+    constexpr int NT = 32 * WM * WN, NST = ring(WM * WN, BN);
     constexpr int WTM = BM / WM, WTN = BN / WN, MI = WTM / 8, NI = WTN / 8;
     constexpr int LA = BM * BK / NT, LB = BN * BK / NT;
-    static_assert(LA >= 1 && LB >= 1 && BM + BN <= NT, "tile shape");
+    static_assert(LA >= 1 && LB >= 1 && NT % BM == 0 && NT % BK == 0, "tile shape");
     extern __shared__ double dsm[];
     double(*As)[BK][BM + PAD] = reinterpret_cast<double(*)[BK][BM + PAD]>(dsm);
-    double(*Bs)[BK][BN + PAD] = reinterpret_cast<double(*)[BK][BN + PAD]>(dsm + 2 * BK * (BM + PAD));
-    __shared__ i64 offM[BM], offN[BN], offKA[2][BK], offKB[2][BK];
+    double(*Bs)[BK][BN + PAD] = reinterpret_cast<double(*)[BK][BN + PAD]>(dsm + NST * BK * (BM + PAD));
+    __shared__ i64 offM[BM], offN[BN], offKA[NST][BK], offKB[NST][BK];
     __shared__ TaskDev tk;
-    __shared__ SegDev sg;
+    __shared__ SegDev sgs[2];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = warp % WM, wn = warp / WM;
     const TileDev tl = tiles[blockIdx.x];
-    if (tid == 0) tk = tasks[tl.task];
+    copy_entry(&tk, tasks + tl.task);
     __syncthreads();
+    copy_entry(&sgs[0], segs + tk.seg0);
     const i64 m0 = (i64)tl.mt * BM, n0 = (i64)tl.nt * BN;
     double acc[MI][NI][2];
 #pragma unroll
     for (int i = 0; i < MI; i++)
 #pragma unroll
         for (int j = 0; j < NI; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
-    double ra[LA], rb[LB];
 
     for (int si = 0; si < tk.nseg; si++) {
         __syncthreads();
-        if (tid == 0) sg = segs[tk.seg0 + si];
-        __syncthreads();
+        const SegDev &sg = sgs[si & 1];
+        // the next segment's entry travels with this one's first stage
+        if (si + 1 < tk.nseg && tid < (int)sizeof(SegDev) / 8)
+            stage_cp(reinterpret_cast<double *>(&sgs[(si + 1) & 1]) + tid,
+                     reinterpret_cast<const double *>(segs + tk.seg0 + si + 1) + tid, true);
         i64 kb = tl.k_lo - sg.kstart, ke = tl.k_hi - sg.kstart;
         if (kb < 0) kb = 0;
         if (ke > sg.K) ke = sg.K;
-        if (kb >= ke) continue;
-        if (tid < BM) {
-            i64 m = m0 + tid;
-            offM[tid] = (m < tk.M) ? sg.baseA + decode1(m, tk.nm, tk.mExt, sg.mSA) : -1;
-        } else if (tid < BM + BN) {
-            i64 n = n0 + tid - BM;
-            offN[tid - BM] = (n < tk.N) ? sg.baseB + decode1(n, tk.nn, tk.nExt, sg.nSB) : -1;
+        if (kb >= ke) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            continue;
+        }
+        for (int j = tid; j < BM + BN; j += NT) {
+            if (j < BM) {
+                const i64 m = m0 + j;
+                offM[j] = (m < tk.M) ? sg.baseA + decode1(m, tk.nm, tk.mExt, sg.mSA) : -1;
+            } else {
+                const i64 n = n0 + j - BM;
+                offN[j - BM] = (n < tk.N) ? sg.baseB + decode1(n, tk.nn, tk.nExt, sg.nSB) : -1;
+            }
         }
         const int nst = (int)((ke - kb + BK - 1) / BK);
-        auto decodeK = [&](int s, int buf) {
-            if (tid < BK) {
-                i64 k = kb + (i64)s * BK + tid;
-                if (k < ke) {
-                    i64 a = 0, b = 0, x = k;
-                    for (int u = 0; u < sg.nk - 1; u++) {
-                        const i64 e = sg.kExt[u];
-                        const i64 q = (x <= 0x7fffffffLL && e <= 0x7fffffffLL) ? (i64)((unsigned)x / (unsigned)e)
-                                                                               : x / e;
-                        const i64 r = x - q * e;
-                        a += r * sg.kSA[u];
-                        b += r * sg.kSB[u];
-                        x = q;
+        // operand offsets of index j of K stage s, into ring slot s % NST
+        auto decodeK = [&](int s, int j) {
+            const i64 k = kb + (i64)s * BK + j;
+            i64 a = -1, b = -1;
+            if (k < ke) {
+                a = b = 0;
+                i64 x = k;
+                for (int u = 0; u < sg.nk - 1; u++) {
+                    const i64 e = sg.kExt[u];
+                    const i64 q = (x <= 0x7fffffffLL && e <= 0x7fffffffLL) ? (i64)((unsigned)x / (unsigned)e) : x / e;
+                    const i64 r = x - q * e;
+                    a += r * sg.kSA[u];
+                    b += r * sg.kSB[u];
+                    x = q;
+                }
+                if (sg.nk > 0) {  // the last unit takes the remaining quotient
+                    a += x * sg.kSA[sg.nk - 1];
+                    b += x * sg.kSB[sg.nk - 1];
+                }
+            }
+            offKA[s % NST][j] = a;
+            offKB[s % NST][j] = b;
+        };
+        // one contracted unit: offsets in a constant step, no table
+        const bool afast = sg.aMfast, bfast = sg.bKfast, lin = sg.nk == 1;
+        const i64 ksa = sg.kSA[0], ksb = sg.kSB[0];
+        const int kend = (int)(ke - kb);
+        auto put_a = [&](int buf, int k, int m, i64 om, bool in, i64 ok) {
+            stage_cp(&As[buf][k][m], in ? A + om + ok : A, in);
+        };
+        auto put_b = [&](int buf, int k, int n, i64 on, bool in, i64 ok) {
+            stage_cp(&Bs[buf][k][n], in ? B + on + ok : B, in);
+        };
+        auto issue = [&](int s) {
+            if (s < nst) {
+                const int buf = s % NST, k0 = s * BK;
+                if (afast) {  // a thread keeps its row (BM divides NT)
+                    const int m = tid % BM;
+                    const i64 om = offM[m];
+#pragma unroll
+                    for (int i = 0; i < LA; i++) {
+                        const int k = tid / BM + i * (NT / BM);
+                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksa : offKA[buf][k]);
                     }
-                    if (sg.nk > 0) {  // the last unit takes the remaining quotient
-                        a += x * sg.kSA[sg.nk - 1];
-                        b += x * sg.kSB[sg.nk - 1];
+                } else {  // a thread keeps its contracted index
+                    const int k = tid % BK;
+                    const i64 ok = lin ? (kb + k0 + k) * ksa : offKA[buf][k];
+#pragma unroll
+                    for (int i = 0; i < LA; i++) {
+                        const int m = tid / BK + i * (NT / BK);
+                        const i64 om = offM[m];
+                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, ok);
                     }
-                    offKA[buf][tid] = a;
-                    offKB[buf][tid] = b;
+                }
+                if (bfast) {
+                    const int k = tid % BK;
+                    const i64 ok = lin ? (kb + k0 + k) * ksb : offKB[buf][k];
+#pragma unroll
+                    for (int i = 0; i < LB; i++) {
+                        const int n = tid / BK + i * (NT / BK);
+                        const i64 on = offN[n];
+                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, ok);
+                    }
                 } else {
-                    offKA[buf][tid] = -1;
-                    offKB[buf][tid] = -1;
+#pragma unroll
+                    for (int i = 0; i < LB; i++) {
+                        const int e = tid + i * NT, n = e % BN, k = e / BN;
+                        const i64 on = offN[n];
+                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksb : offKB[buf][k]);
+                    }
                 }
             }
+            asm volatile("cp.async.commit_group;" ::: "memory");  // an empty group past the end keeps the count
         };
-        auto loadRegs = [&](int buf) {
-#pragma unroll
-            for (int i = 0; i < LA; i++) {
-                int e = tid + i * NT, m, k;
-                if (sg.aMfast) {
-                    m = e % BM;
-                    k = e / BM;
-                } else {
-                    k = e % BK;
-                    m = e / BK;
-                }
-                i64 om = offM[m], ok = offKA[buf][k];
-                ra[i] = (om >= 0 && ok >= 0) ? __ldg(A + om + ok) : 0.0;
-            }
-#pragma unroll
-            for (int i = 0; i < LB; i++) {
-                int e = tid + i * NT, n, k;
-                if (sg.bKfast) {
-                    k = e % BK;
-                    n = e / BK;
-                } else {
-                    n = e % BN;
-                    k = e / BN;
-                }
-                i64 on = offN[n], ok = offKB[buf][k];
-                rb[i] = (on >= 0 && ok >= 0) ? __ldg(B + on + ok) : 0.0;
-            }
-        };
-        auto storeRegs = [&](int buf) {
-#pragma unroll
-            for (int i = 0; i < LA; i++) {
-                int e = tid + i * NT;
-                if (sg.aMfast) As[buf][e / BM][e % BM] = ra[i];
-                else As[buf][e % BK][e / BK] = ra[i];
-            }
-#pragma unroll
-            for (int i = 0; i < LB; i++) {
-                int e = tid + i * NT;
-                if (sg.bKfast) Bs[buf][e % BK][e / BK] = rb[i];
-                else Bs[buf][e / BN][e % BN] = rb[i];
-            }
-        };
-        decodeK(0, 0);
+        if (!lin && tid < BK * NST) decodeK(tid / BK, tid % BK);
         __syncthreads();
-        loadRegs(0);
+#pragma unroll
+        for (int s = 0; s < NST - 1; s++) issue(s);
         for (int s = 0; s < nst; s++) {
-            const int buf = s & 1;
-            storeRegs(buf);
-            if (s + 1 < nst) decodeK(s + 1, buf ^ 1);
-            __syncthreads();
-            if (s + 1 < nst) loadRegs(buf ^ 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(NST - 2) : "memory");
+            __syncthreads();  // stage s is complete; slot s - 1 and its offsets are free
+            issue(s + NST - 1);
+            if (!lin && tid < BK && s + NST < nst) decodeK(s + NST, tid);
+            const int buf = s % NST;
 #pragma unroll
             for (int kk = 0; kk < BK / 4; kk++) {
                 const int kr = kk * 4 + (lane & 3);
@@ -183,6 +220,7 @@ __global__ void __launch_bounds__(NT, 2) k_contract(const double *__restrict__ A
             }
         }
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     const int rl = lane >> 2, cl = 2 * (lane & 3);
     if (tl.part >= 0) {
@@ -197,12 +235,14 @@ __global__ void __launch_bounds__(NT, 2) k_contract(const double *__restrict__ A
             }
         return;
     }
-    if (tid < BM) {
-        i64 m = m0 + tid;
-        offM[tid] = (m < tk.M) ? tk.baseC + decode1(m, tk.nm, tk.mExt, tk.mSC) : -1;
-    } else if (tid < BM + BN) {
-        i64 n = n0 + tid - BM;
-        offN[tid - BM] = (n < tk.N) ? decode1(n, tk.nn, tk.nExt, tk.nSC) : -1;
+    for (int j = tid; j < BM + BN; j += NT) {
+        if (j < BM) {
+            const i64 m = m0 + j;
+            offM[j] = (m < tk.M) ? tk.baseC + decode1(m, tk.nm, tk.mExt, tk.mSC) : -1;
+        } else {
+            const i64 n = n0 + j - BM;
+            offN[j - BM] = (n < tk.N) ? decode1(n, tk.nn, tk.nExt, tk.nSC) : -1;
+        }
     }
     __syncthreads();
 #pragma unroll
@@ -274,8 +314,8 @@ int timing_event(cudaEvent_t *e) {
 }
 }  // namespace
 
-const int TILE_BM[4] = {128, 128, 64, 64};
-const int TILE_BN[4] = {64, 32, 128, 64};
+const int TILE_BM[NTILE] = {128, 128, 64, 64, 128};
+const int TILE_BN[NTILE] = {64, 32, 128, 64, 16};
 
 int contract_timing(int enable) {
     timing().on = enable != 0;
@@ -377,7 +417,7 @@ int tune_plan(const ContractPlan *p, const double *A, const double *B, const Con
     CPSD_TRY(cuda_check(cudaEventCreate(&e1), "event"));
     float best_ms = 1e30f;
     int rc = CPSD_OK;
-    for (int c = 0; c < 4 && rc == CPSD_OK; c++) {
+    for (int c = 0; c < NTILE && rc == CPSD_OK; c++) {
         const ContractPlan *q = p;
         if (c != p->cfg) {
             auto v = std::make_unique<ContractPlan>();
@@ -440,6 +480,35 @@ int launch_contract(const ContractPlan *p, const double *A, const double *B, dou
 }
 
 namespace {
+// kernel attributes of the tile shapes (of the current device when `again`)
+int tile_attrs(bool again = false) {
+    static std::atomic<bool> done{false};
+    if (done.load(std::memory_order_acquire) && !again) return CPSD_OK;
+    auto one = [](const void *k, int bytes) {
+        return cuda_check(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "smem attr");
+    };
+    CPSD_TRY(one((const void *)k_contract<128, 64, 4, 2>, smem_bytes<128, 64, 8>()));
+    CPSD_TRY(one((const void *)k_contract<128, 32, 4, 1>, smem_bytes<128, 32, 4>()));
+    CPSD_TRY(one((const void *)k_contract<64, 128, 2, 4>, smem_bytes<64, 128, 8>()));
+    CPSD_TRY(one((const void *)k_contract<64, 64, 2, 2>, smem_bytes<64, 64, 4>()));
+    CPSD_TRY(one((const void *)k_contract<128, 16, 4, 1>, smem_bytes<128, 16, 4>()));
+    done.store(true, std::memory_order_release);
+    return CPSD_OK;
+}
+void run_tiles(int cfg, int ntiles, const double *A, const double *B, double *C, const TaskDev *tk, const SegDev *sg,
+               const TileDev *tl, double alpha, double *part) {
+#define CPSD_TILE(BM, BN, WM, WN)                                                                                \
+    k_contract<BM, BN, WM, WN><<<ntiles, 32 * WM * WN, smem_bytes<BM, BN, WM * WN>(), stream()>>>(A, B, C, tk, sg, tl, alpha, part)
+    switch (cfg) {
+    case 0: CPSD_TILE(128, 64, 4, 2); break;
+    case 1: CPSD_TILE(128, 32, 4, 1); break;
+    case 2: CPSD_TILE(64, 128, 2, 4); break;
+    case 3: CPSD_TILE(64, 64, 2, 2); break;
+    default: CPSD_TILE(128, 16, 4, 1); break;
+    }
+#undef CPSD_TILE
+}
+
 int launch_tiles(const ContractPlan *p, const double *A, const double *B, double *C, double alpha) {
     CPSD_TRY(const_cast<ContractPlan *>(p)->upload());
     const int bm = TILE_BM[p->cfg], bn = TILE_BN[p->cfg];
@@ -454,36 +523,8 @@ int launch_tiles(const ContractPlan *p, const double *A, const double *B, double
         timing().shape.push_back({p->ntasks, p->nsegs, p->ntiles, p->cfg});
         CPSD_TRY(cuda_check(cudaEventRecord(e0, stream()), "event record"));
     }
-    static std::atomic<bool> attr_set{false};
-    if (!attr_set) {
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<128, 64, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<128, 64>()), "smem attr"));
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<128, 32, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<128, 32>()), "smem attr"));
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<64, 128, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<64, 128>()), "smem attr"));
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<64, 64, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<64, 64>()), "smem attr"));
-        attr_set = true;
-    }
-    switch (p->cfg) {
-    case 0:
-        k_contract<128, 64, 4, 2><<<p->ntiles, NT, smem_bytes<128, 64>(), stream()>>>(
-            A, B, C, p->d_tasks, p->d_segs, p->d_tiles, alpha, part);
-        break;
-    case 1:
-        k_contract<128, 32, 4, 2><<<p->ntiles, NT, smem_bytes<128, 32>(), stream()>>>(
-            A, B, C, p->d_tasks, p->d_segs, p->d_tiles, alpha, part);
-        break;
-    case 2:
-        k_contract<64, 128, 2, 4><<<p->ntiles, NT, smem_bytes<64, 128>(), stream()>>>(
-            A, B, C, p->d_tasks, p->d_segs, p->d_tiles, alpha, part);
-        break;
-    default:
-        k_contract<64, 64, 2, 4><<<p->ntiles, NT, smem_bytes<64, 64>(), stream()>>>(
-            A, B, C, p->d_tasks, p->d_segs, p->d_tiles, alpha, part);
-        break;
-    }
+    CPSD_TRY(tile_attrs());
+    run_tiles(p->cfg, p->ntiles, A, B, C, p->d_tasks, p->d_segs, p->d_tiles, alpha, part);
     count_launch();
     ctx().flops += p->flops;
     if (e1) CPSD_TRY(cuda_check(cudaEventRecord(e1, stream()), "event record"));
@@ -541,14 +582,7 @@ int noalloc_setup(unsigned char **base) {
         }
         void *p = nullptr;
         CPSD_TRY(cuda_check(cudaGetSymbolAddress(&p, g_noalloc_scratch), "cudaGetSymbolAddress(noalloc scratch)"));
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<128, 64, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<128, 64>()), "smem attr"));
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<128, 32, 4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<128, 32>()), "smem attr"));
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<64, 128, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<64, 128>()), "smem attr"));
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(k_contract<64, 64, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 smem_bytes<64, 64>()), "smem attr"));
+        CPSD_TRY(tile_attrs(true));
         g_noalloc_base[dev].store((unsigned char *)p);
     }
     *base = g_noalloc_base[dev].load();
@@ -558,17 +592,21 @@ int noalloc_setup(unsigned char **base) {
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 }  // namespace
 
-size_t contract_noalloc_bytes(const ContractPlan *p) {
-    if (p->empty) return 0;
+size_t contract_noalloc_bytes(const ContractPlan *plan) {
+    if (plan->empty) return 0;
+    const ContractPlan *p;
+    if (plan_fixed(plan, &p) != CPSD_OK) return 0;
     const size_t tile = (size_t)TILE_BM[p->cfg] * TILE_BN[p->cfg] * sizeof(double);
     return align256(p->h_tasks.size() * sizeof(TaskDev)) + align256(p->h_segs.size() * sizeof(SegDev)) +
            align256(p->h_tiles.size() * sizeof(TileDev)) + align256(p->h_reduce.size() * sizeof(int)) +
            align256((size_t)p->nparts * tile);
 }
 
-int launch_contract_noalloc(const ContractPlan *p, const double *A, const double *B, double *C, double alpha) {
-    if (p->empty) return CPSD_OK;
-    const size_t need = contract_noalloc_bytes(p);
+int launch_contract_noalloc(const ContractPlan *plan, const double *A, const double *B, double *C, double alpha) {
+    if (plan->empty) return CPSD_OK;
+    const size_t need = contract_noalloc_bytes(plan);
+    const ContractPlan *p;
+    CPSD_TRY(plan_fixed(plan, &p));
     if (need > (size_t)CPSD_NOALLOC_SCRATCH_BYTES)
         return set_error(CPSD_EARG, "contraction needs " + std::to_string(need) +
                                         " bytes of scratch; the no-allocation entry point holds at most " +
@@ -600,20 +638,7 @@ int launch_contract_noalloc(const ContractPlan *p, const double *A, const double
         timing().shape.push_back({p->ntasks, p->nsegs, p->ntiles, p->cfg});
         CPSD_TRY(cuda_check(cudaEventRecord(e0, stream()), "event record"));
     }
-    switch (p->cfg) {
-    case 0:
-        k_contract<128, 64, 4, 2><<<p->ntiles, NT, smem_bytes<128, 64>(), stream()>>>(A, B, C, tk, sg, tl, alpha, part);
-        break;
-    case 1:
-        k_contract<128, 32, 4, 2><<<p->ntiles, NT, smem_bytes<128, 32>(), stream()>>>(A, B, C, tk, sg, tl, alpha, part);
-        break;
-    case 2:
-        k_contract<64, 128, 2, 4><<<p->ntiles, NT, smem_bytes<64, 128>(), stream()>>>(A, B, C, tk, sg, tl, alpha, part);
-        break;
-    default:
-        k_contract<64, 64, 2, 4><<<p->ntiles, NT, smem_bytes<64, 64>(), stream()>>>(A, B, C, tk, sg, tl, alpha, part);
-        break;
-    }
+    run_tiles(p->cfg, p->ntiles, A, B, C, tk, sg, tl, alpha, part);
     count_launch();
     ctx().flops += p->flops;
     if (e1) CPSD_TRY(cuda_check(cudaEventRecord(e1, stream()), "event record"));

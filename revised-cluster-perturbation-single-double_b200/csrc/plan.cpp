@@ -93,16 +93,82 @@ int EnergyPlan::upload() {
     return CPSD_OK;
 }
 
-// Tile shape, tiles and split-K groups of a plan whose tasks and segments
-// are built: the shape with the least estimated time counting the padded
-// tensor-pipe work (FP64 ~35 TFLOP/s) and the operand re-reads (~6 TB/s),
-// or force_cfg when it is >= 0; split-K so that small outputs with long K
-// still fill the GPU
-void finish_plan(ContractPlan *plan, std::vector<TaskDev> tasks, std::vector<SegDev> dsegs, int force_cfg) {
+namespace {
+// Tile shape (or force_cfg when it is >= 0) and K parts of a launch: those with
+// the least estimated time.  An SM holds two or three CTAs,
+// so tiles run in waves of that many on 148 SMs; a full SM reaches the part
+// TILE_EFF of 37 TFLOP/s on the padded work, one CTA alone TILE_LONE of it
+// (measured on particle ladders of 8 to 300 columns); a tile starts in 2.5 us,
+// each K segment of it in 2 us; split tiles add the reduction's launch and
+// their partial sums' traffic; nothing beats the operand re-reads at 6 TB/s.
+// A part keeps at least two stages.  (The parts used to be as many as fill 592
+// tiles with 256 deep parts, whatever the wave: 70 tiles of the C1 nmo-71
+// ladder made 630, two full waves and a tenth of a third, 299 us, now 240; 36
+// tiles of a C2v nmo-48 ring stayed 36, 37 us, now 24 with its reduction.)
+constexpr i64 TILE_CTAS[NTILE] = {2, 3, 2, 3, 2};
+constexpr double TILE_EFF[NTILE] = {0.66, 0.62, 0.64, 0.74, 0.45}, TILE_LONE[NTILE] = {0.42, 0.25, 0.42, 0.28, 0.17};
+constexpr i64 MINPART = 32;
+void choose_tiles(const std::vector<TaskDev> &tasks, int force_cfg, int *cfg_out, i64 *split_out) {
+    constexpr i64 SMS = 148;
+    auto parts_of = [&](const TaskDev &tk, i64 ns) { return std::min(ns, std::max<i64>(1, tk.Ktot / MINPART)); };
+    int cfg = 0;
+    i64 split = 1;
+    double best = 1e300;
+    for (int c = 0; c < NTILE; c++) {
+        if (force_cfg >= 0 && c != force_cfg) continue;
+        const i64 bm = TILE_BM[c], bn = TILE_BN[c], slots = TILE_CTAS[c] * SMS;
+        // time of a K stage of 16 with r CTAs on the SM
+        auto stage = [&](i64 r) {
+            return (double)r * 2.0 * (double)(bm * bn) * 16 / (37e12 / SMS) / std::min(TILE_EFF[c], (double)r * TILE_LONE[c]);
+        };
+        double by = 0;
+        i64 maxk = 0, base = 0;
+        for (auto &tk : tasks) {
+            const double mt = (double)((tk.M + bm - 1) / bm), nt = (double)((tk.N + bn - 1) / bn);
+            by += 8.0 * (double)tk.Ktot * ((double)tk.M * nt + (double)tk.N * mt);
+            maxk = std::max(maxk, tk.Ktot);
+            base += (i64)(mt * nt);
+        }
+        for (i64 ns = 1; ns <= 64; ns++) {
+            if (ns > 1 && (ns > std::max<i64>(1, maxk / MINPART) || base * ns > 6 * SMS)) break;
+            i64 tiles = 0;
+            double work = 0;  // stages of all tiles
+            i64 longest = 0, nseg = 1;
+            for (auto &tk : tasks) {
+                const i64 np = parts_of(tk, ns), st = ((tk.Ktot + np - 1) / np + 15) / 16;
+                const i64 n = ((tk.M + bm - 1) / bm) * ((tk.N + bn - 1) / bn) * np;
+                tiles += n;
+                work += (double)(n * st);
+                longest = std::max(longest, st);
+                nseg = std::max<i64>(nseg, (tk.nseg + np - 1) / np);
+            }
+            const double start = 2.5e-6 + 2e-6 * (double)nseg;
+            const i64 full = tiles / slots, rest = tiles % slots;
+            const double st = std::max(work / (double)std::max<i64>(tiles, 1), full ? 0.0 : (double)longest);
+            double t = (double)full * (start + st * stage(TILE_CTAS[c]));
+            if (rest) t += start + st * stage((rest + SMS - 1) / SMS);
+            t = std::max(t, by / 6e12);
+            if (ns > 1) t += 3e-6 + (double)tiles * (double)(bm * bn) * 16 / 4e12;
+            if (t < best * 0.999) {
+                best = t;
+                cfg = c;
+                split = ns;
+            }
+        }
+    }
+    *cfg_out = cfg;
+    *split_out = split;
+}
+
+// The choice of the entry point that allocates nothing.  What it accepts is
+// part of its interface (the partial tiles have to fit its fixed region), so
+// it keeps one rule for good: the shape by padded work and operand re-reads,
+// K parts of at least 256 until 592 tiles are there.
+constexpr i64 FIXED_MINPART = 256;
+void choose_tiles_fixed(const std::vector<TaskDev> &tasks, int *cfg_out, i64 *split_out) {
     int cfg = 0;
     double best = 1e300;
     for (int c = 0; c < 4; c++) {
-        if (force_cfg >= 0 && c != force_cfg) continue;
         double fl = 0, by = 0;
         for (auto &tk : tasks) {
             double mt = (double)((tk.M + TILE_BM[c] - 1) / TILE_BM[c]), nt = (double)((tk.N + TILE_BN[c] - 1) / TILE_BN[c]);
@@ -115,22 +181,31 @@ void finish_plan(ContractPlan *plan, std::vector<TaskDev> tasks, std::vector<Seg
             cfg = c;
         }
     }
+    i64 mn_tiles = 0;
+    for (auto &tk : tasks)
+        mn_tiles += ((tk.M + TILE_BM[cfg] - 1) / TILE_BM[cfg]) * ((tk.N + TILE_BN[cfg] - 1) / TILE_BN[cfg]);
+    const i64 target = 4 * 148;
+    *cfg_out = cfg;
+    *split_out = (mn_tiles >= target || mn_tiles == 0) ? 1 : std::min<i64>(64, (target + mn_tiles - 1) / mn_tiles);
+}
+}  // namespace
+
+// Tiles and split-K groups of a plan whose tasks and segments are built
+void finish_plan(ContractPlan *plan, std::vector<TaskDev> tasks, std::vector<SegDev> dsegs, int force_cfg, bool fixed) {
+    int cfg;
+    i64 split;
+    if (fixed) choose_tiles_fixed(tasks, &cfg, &split);
+    else choose_tiles(tasks, force_cfg, &cfg, &split);
+    const i64 minpart = fixed ? FIXED_MINPART : MINPART;
     const i64 TBM = TILE_BM[cfg], TBN = TILE_BN[cfg];
     plan->cfg = cfg;
-    // tiles, with split-K so that small outputs with long K still fill the GPU
     std::vector<TileDev> tiles;
     std::vector<int> red;
-    i64 mn_tiles = 0;
-    for (auto &tk : tasks) mn_tiles += ((tk.M + TBM - 1) / TBM) * ((tk.N + TBN - 1) / TBN);
-    const i64 target = 4 * 148;
     i64 part = 0;
     for (int ti = 0; ti < (int)tasks.size(); ti++) {
         const TaskDev &tk = tasks[ti];
         i64 mt = (tk.M + TBM - 1) / TBM, nt = (tk.N + TBN - 1) / TBN;
-        i64 want = (mn_tiles >= target) ? 1 : (target + mn_tiles - 1) / mn_tiles;
-        i64 maxsplit = std::max<i64>(1, tk.Ktot / 256);
-        i64 ns = std::min(want, maxsplit);
-        if (ns > 64) ns = 64;
+        const i64 ns = std::min(split, std::max<i64>(1, tk.Ktot / minpart));
         for (i64 a = 0; a < mt; a++)
             for (i64 b = 0; b < nt; b++) {
                 if (ns > 1) {
@@ -460,6 +535,20 @@ int plan_contract(const Desc &d1, const char *t1, const Desc &d2, const char *t2
     finish_plan(plan.get(), std::move(tasks), std::move(dsegs));
     *out = plan.get();
     cache[key] = std::move(plan);
+    return CPSD_OK;
+}
+
+int plan_fixed(const ContractPlan *p, const ContractPlan **out) {
+    static std::mutex m;
+    std::lock_guard<std::mutex> lock(m);
+    static std::map<const ContractPlan *, std::unique_ptr<ContractPlan>> cache;
+    auto &q = cache[p];
+    if (!q) {
+        q = std::make_unique<ContractPlan>();
+        q->flops = p->flops;
+        finish_plan(q.get(), p->h_tasks, p->h_segs, -1, true);
+    }
+    *out = q.get();
     return CPSD_OK;
 }
 

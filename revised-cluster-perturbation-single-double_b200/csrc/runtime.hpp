@@ -162,9 +162,10 @@ struct TileDev {
     i64 part;            // partial slot (split-K) or -1
 };
 
-// tile shapes of the contraction kernel: BM x BN = 128x64, 128x32, 64x128, 64x64
-extern const int TILE_BM[4];
-extern const int TILE_BN[4];
+// tile shapes of the contraction kernel: BM x BN = 128x64, 128x32, 64x128, 64x64, 128x16
+constexpr int NTILE = 5;
+extern const int TILE_BM[NTILE];
+extern const int TILE_BN[NTILE];
 
 struct ContractPlan {
     bool empty = true;
@@ -198,9 +199,13 @@ int plan_contract(const Desc &d1, const char *t1, const Desc &d2, const char *t2
                   const char *t3, const Batch &batch, const ContractPlan **out);
 // tiles of a plan whose tasks and segments are built (force_cfg >= 0: that
 // tile shape instead of the cost model's)
-void finish_plan(ContractPlan *plan, std::vector<TaskDev> tasks, std::vector<SegDev> dsegs, int force_cfg = -1);
+// (fixed: the choice of the entry point that allocates nothing)
+void finish_plan(ContractPlan *plan, std::vector<TaskDev> tasks, std::vector<SegDev> dsegs, int force_cfg = -1,
+                 bool fixed = false);
+// the plan with the tiles of the entry point that allocates nothing
+int plan_fixed(const ContractPlan *p, const ContractPlan **out);
 // empirical tile-shape choice (off by default): with it on, the first
-// launch of each FP64 tile plan times the four tile shapes on a scratch
+// launch of each FP64 tile plan times the tile shapes on a scratch
 // copy of the output and later launches use the fastest
 int set_tile_autotune(int on);
 int tile_autotune_stats(int64_t *tuned, int64_t *changed);
@@ -251,7 +256,7 @@ int launch_contract(const ContractPlan *p, const double *A, const double *B, dou
 int launch_contract_noalloc(const ContractPlan *p, const double *A, const double *B, double *C, double alpha);
 size_t contract_noalloc_bytes(const ContractPlan *p);
 // CUDA-event record of one more launch in the timing buffer (when timing is
-// on): kind 0-3 DMMA tile shapes, 10 / 11 digit slicing of A / B, 12 digit
+// on): kind 0-4 DMMA tile shapes, 10 / 11 digit slicing of A / B, 12 digit
 // GEMM, 20 / 21 narrow-output kernels (rows / K), 22 short-K kernel (tasks,
 // tiles, output elements), 23 row-dot kernel (tasks, warps, output
 // elements), 30 / 31 Davidson step /
