@@ -175,7 +175,7 @@ constexpr int GL = DAV_MAXD + 1;
 // a thread is the same in all rounds.  (Indexing the pairs anew took 1250
 // cycles a round; roots, divisions and the index arithmetic 2000.)
 __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n) {
-    __shared__ double cs[DAV_MAXD / 2], sn[DAV_MAXD / 2];
+    __shared__ double cs[DAV_MAXD / 2], sn[DAV_MAXD / 2], tn[DAV_MAXD / 2];
     __shared__ int rotate;  // last round that saw an element above the threshold
     const int tid = threadIdx.x;
     const int m = (n + 1) & ~1, half = m / 2;
@@ -273,6 +273,7 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
             if (d != 0.0 && ((d > 0.0) != (b > 0.0))) s = -s;
             cs[tid] = keep ? 1.0 : u * ru;
             sn[tid] = keep ? 0.0 : s;
+            tn[tid] = keep ? 0.0 : s * ru;  // s / c
         }
         __syncthreads();
         if (rotate != round) break;
@@ -283,10 +284,14 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
                 const double ck = cs[k0], sk = sn[k0];
                 const double t00 = cl * b00 - sl * b01, t01 = sl * b00 + cl * b01;
                 const double t10 = cl * b10 - sl * b11, t11 = sl * b10 + cl * b11;
-                B[w00] = ck * t00 - sk * t10;
-                B[w01] = dia ? 0.0 : ck * t01 - sk * t11;  // annihilated (or negligible) element
+                const double tk = tn[k0];
+                // a pair's own block: a_pp - t a_pq, a_qq + t a_pq, so that c^2
+                // + s^2 being 1 to rounding only does not add up in the
+                // eigenvalues, and an annihilated (or negligible) element
+                B[w00] = dia ? fma(-tk, b01, b00) : ck * t00 - sk * t10;
+                B[w01] = dia ? 0.0 : ck * t01 - sk * t11;
                 B[w10] = dia ? 0.0 : sk * t00 + ck * t10;
-                B[w11] = sk * t01 + ck * t11;
+                B[w11] = dia ? fma(tk, b01, b11) : sk * t01 + ck * t11;
             }
         } else {
             if (live0) {

@@ -8,7 +8,9 @@ order in the residual (1e-10 here) and rounding leaves about n eps |A| (n up
 to 4000, |A| of a few Eh), so 1e-11 Eh bounds both.  The DIIS loop against
 the oracle's, which takes the same steps: rounding differences of 1e-16 grow
 through the extrapolations of a converging loop, 1e-9 of the amplitudes'
-size, the loop's own tolerance being 1e-7.
+size, the loop's own tolerance being 1e-7.  Nine and more roots get a basis of
+32: in one of 20 they take 86 to over 300 cycles from seed to seed (and end at
+the cycle limit at some, as one-CTA steps do), a count that rounding decides.
 """
 import numpy as np
 import pytest
@@ -32,7 +34,7 @@ pytestmark = pytest.mark.gpu
 ])
 def test_cis_roots_match_dense(nmo, nocc_a, nirrep, roots):
     s = synth.System(nmo=nmo, nocc_a=nocc_a, nocc_b=nocc_a - 2, nirrep=nirrep, seed=3, roots=roots, skip_abcd=True,
-                     run_opts=dict(lowest=1, davidson_conv=10, davidson_cyc=300, davidson_dim=20 if roots < 10 else 32))
+                     run_opts=dict(lowest=1, davidson_conv=10, davidson_cyc=300, davidson_dim=20 if roots < 9 else 32))
     api.use_torch_stream()
     ints = api.DeviceIntegrals(s)
     om, R, it = api.cis_run(s, api.make_system(s), ints, api.make_params(s))
