@@ -268,22 +268,23 @@ __global__ void __launch_bounds__(256) k_dot_partial(const double *__restrict__ 
     }
     if (threadIdx.x == 0) part[blockIdx.x] = s[0];
 }
-// fixed-order final sum; Neumaier compensation when requested
-__global__ void k_dot_final(const double *__restrict__ part, int np, double *out, int comp) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// final sum by one warp, fixed order; with comp every sum carries its rounding
+// error along (Neumaier per lane, exact two-sums across lanes).  One thread
+// walking the partial sums in global memory took 14 us.
+__global__ void __launch_bounds__(32) k_dot_final(const double *__restrict__ part, int np, double *out, int comp) {
     double s = 0.0, c = 0.0;
-    for (int i = 0; i < np; i++) {
-        double v = part[i];
-        if (comp) {
-            double t = s + v;
-            if (fabs(s) >= fabs(v)) c += (s - t) + v;
-            else c += (v - t) + s;
-            s = t;
-        } else {
-            s += v;
-        }
+    for (int i = threadIdx.x; i < np; i += 32) {
+        const double v = part[i], t = s + v;
+        if (comp) c += fabs(s) >= fabs(v) ? (s - t) + v : (v - t) + s;
+        s = t;
     }
-    *out = s + c;
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v = __shfl_down_sync(0xffffffffu, s, o), t = s + v;
+        const double cv = __shfl_down_sync(0xffffffffu, c, o);
+        if (comp) c += cv + (fabs(s) >= fabs(v) ? (s - t) + v : (v - t) + s);
+        s = t;
+    }
+    if (threadIdx.x == 0) *out = s + c;
 }
 
 int grid_for(i64 n, int threads = 256) {
