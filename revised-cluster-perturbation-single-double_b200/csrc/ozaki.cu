@@ -422,6 +422,67 @@ __global__ void __launch_bounds__(256) k_oz_expo(const OzSliceJob *__restrict__ 
         if (r0 + i < jb.R && rmax[i] != OZ_EXPO_NONE) atomicMax(&expo[jb.eoff + r0 + i], rmax[i]);
 }
 
+// The S digits of four scaled values (|y| < 1) as S words of four bytes, word
+// t holding digit t of y[0..3].  Cutting off digits by truncation leaves the
+// 7-bit fields of |y| 2^(7S) rounded towards zero, under the sign of y; one
+// FP64 addition of 2^(52 - 7S), rounded towards zero, puts exactly that
+// integer into the low mantissa bits.  The fields are then spread to bytes,
+// transposed and given their signs four at a time: 54 integer and 4 FP64
+// instructions for four values of five digits.  (Five rounds of multiply,
+// truncate, subtract and convert were bound by the conversions: 1.86 ms for
+// the 665 M elements of the D2h nmo-200 list, where its traffic takes 1.3.)
+__device__ __forceinline__ uint32_t oz_spread(uint32_t v) {
+    // 14-bit halves, then 7-bit fields, to byte lanes; the top bit of a byte is
+    // left over and masked by the caller
+    const uint32_t w = (v & 0x0000ffffu) | ((v << 2) & 0xffff0000u);
+    return (w & 0x00ff00ffu) | ((w << 1) & 0xff00ff00u);
+}
+// byte permutation whose selector nibbles 8..15 replicate a byte's sign (the
+// __byte_perm intrinsic masks that bit off)
+__device__ __forceinline__ uint32_t oz_signs(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("prmt.b32 %0, %1, %2, 0x00fb;" : "=r"(d) : "r"(a), "r"(b));
+    return d;  // byte 0: sign of a, byte 1: sign of b
+}
+template <int S>
+__device__ __forceinline__ void oz_digits4(const double (&y)[4], uint32_t (&w)[S]) {
+    constexpr double MAGIC = (double)(1ull << (52 - 7 * S));
+    uint32_t lo[4], hi[4], h[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        const double t = __dadd_rz(fabs(y[j]), MAGIC);
+        const uint32_t tl = (uint32_t)__double2loint(t), th = (uint32_t)__double2hiint(t);
+        lo[j] = oz_spread(tl);  // fields 0..3 from below: digits S-1 .. S-4
+        const uint32_t up = __funnelshift_r(tl, th, 28);
+        hi[j] = S > 5 ? oz_spread(up) : up;  // fields 4..: digits S-5 .. 0
+        h[j] = (uint32_t)__double2hiint(y[j]);
+    }
+    // sign of each value over its byte
+    const uint32_t m = __byte_perm(oz_signs(h[0], h[1]), oz_signs(h[2], h[3]), 0x5410);
+    auto field = [&](const uint32_t (&x)[4], int b) {  // byte b of the four words
+        const uint32_t sel = (uint32_t)(b | (b + 4) << 4);
+        return __byte_perm(__byte_perm(x[0], x[1], sel), __byte_perm(x[2], x[3], sel), 0x5410);
+    };
+    auto put = [&](int t, uint32_t v) {
+        v &= 0x7f7f7f7fu;
+        const uint32_t neg = (0x80808080u - v) ^ 0x80808080u;  // -v in every byte, no borrow between them
+        w[t] = (neg & m) | (v & ~m);
+    };
+    if constexpr (S >= 4) {  // 4 x 4 byte transpose
+        const uint32_t a = __byte_perm(lo[0], lo[1], 0x5140), b = __byte_perm(lo[2], lo[3], 0x5140);
+        const uint32_t c = __byte_perm(lo[0], lo[1], 0x7362), d = __byte_perm(lo[2], lo[3], 0x7362);
+        put(S - 1, __byte_perm(a, b, 0x5410));
+        put(S - 2, __byte_perm(a, b, 0x7632));
+        put(S - 3, __byte_perm(c, d, 0x5410));
+        put(S - 4, __byte_perm(c, d, 0x7632));
+#pragma unroll
+        for (int t = 0; t < S - 4; t++) put(t, field(hi, S - 5 - t));
+    } else {
+#pragma unroll
+        for (int t = 0; t < S; t++) put(t, field(lo, S - 1 - t));
+    }
+}
+
 // pass 2: the S digit tiles of stage blockIdx.y, written as 16-byte rows of
 // the core matrices; rows and columns beyond the group's extents get zero
 // digits
@@ -457,15 +518,13 @@ __global__ void __launch_bounds__(256) k_oz_slice(const OzSliceJob *__restrict__
 #pragma unroll
         for (int u = 0; u < NU; u++)
 #pragma unroll
-            for (int q = 0; q < 16; q++) {
-                double y = x[u][q] * sc1 * sc2;
+            for (int q = 0; q < 16; q += 4) {
+                const double y[4] = {x[u][q] * sc1 * sc2, x[u][q + 1] * sc1 * sc2, x[u][q + 2] * sc1 * sc2,
+                                     x[u][q + 3] * sc1 * sc2};
+                uint32_t d[S];
+                oz_digits4<S>(y, d);
 #pragma unroll
-                for (int t = 0; t < S; t++) {
-                    y *= 128.0;
-                    const double qd = trunc(y);
-                    y -= qd;
-                    w[u][t][q >> 2] |= ((uint32_t)(uint8_t)(int8_t)(int)qd) << (8 * (q & 3));
-                }
+                for (int t = 0; t < S; t++) w[u][t][q >> 2] = d[t];
             }
     }
 #pragma unroll
