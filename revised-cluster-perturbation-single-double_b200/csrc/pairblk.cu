@@ -9,7 +9,10 @@
 // q stay in registers for the whole block, those over p are finished within
 // the strip.  Strips have a leading dimension of 4 mod 16 doubles, so that
 // both fragment shapes (8 p x 4 q and 8 q x 4 p) fall on different banks.
-// A warp only reads what it copied itself.
+// A warp only reads what it copied itself.  C2v nmo 151 (373 MB of list): 152 us a
+// launch; 204 us with the copies' addresses formed anew for every element (64
+// instructions per 32 elements, issue-bound) and the strip's other loads not
+// ahead; expansion and row-dot contraction took 811 us.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -29,15 +32,13 @@ __device__ __forceinline__ void pb_dmma(double (&c)[2], double a, double b) {
                  : "d"(a), "d"(b));
 }
 // 8-byte copy, or zero fill without reading the source
-__device__ __forceinline__ void pb_cp(double *dst, const double *src, bool read) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                 "l"(src), "r"(read ? 8 : 0)
-                 : "memory");
+__device__ __forceinline__ void pb_cp(uint32_t dst, const double *src, bool read) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(read ? 8 : 0) : "memory");
 }
 
 template <int FT>
 constexpr int pb_ld() {
-    return FT * 8 + 4;  // FT even: 4 mod 16
+    return FT * 8 + 4;  // FT a multiple of 4: 4 mod 16
 }
 template <int FT>
 constexpr int pb_strip() {
@@ -64,6 +65,7 @@ __device__ void pb_block(const PairGroup &g, const double *__restrict__ V, const
     constexpr int LD = pb_ld<FT>();
     const int lane = threadIdx.x & 31, hi = lane >> 2, lo = lane & 3;
     const bool dop = g.ncp > 0, doq = g.ncq > 0;
+    const uint32_t ring_at = (uint32_t)__cvta_generic_to_shared(ring + lane);
     for (int p0 = 0; p0 < g.np; p0 += FT * 8) {
         const int np = min(FT * 8, g.np - p0);
         double acc[FT][2], bp[2 * FT];
@@ -80,32 +82,44 @@ __device__ void pb_block(const PairGroup &g, const double *__restrict__ V, const
             const int lim = g.tri ? min(np, 8 * s + 7 - p0) : np;
             return lim <= 0 ? 0 : (lim + 7) & ~7;
         };
+        // whole runs of 32 rows, zero-filled past the strip's last row (a
+        // strip is FT * 8 rows wide, a multiple of 32); addresses go on by the
+        // length of a run, three or four instructions a copy
         auto issue = [&](int s) {
             if (s < s1) {
-                const int pr = rows(s);
-                double *d = ring + (s % PST) * pb_strip<FT>();
+                const int pr = rows(s), q0 = 8 * s;
+                uint32_t d = ring_at + (uint32_t)((s % PST) * pb_strip<FT>()) * 8;
+                const double *src = V + (g.tri ? (i64)q0 * (q0 - 1) / 2 : (i64)q0 * g.np) + p0 + lane;
 #pragma unroll
                 for (int e = 0; e < 8; e++) {
-                    const int q = 8 * s + e;
-                    const double *src = V + (g.tri ? (i64)q * (q - 1) / 2 : (i64)q * g.np) + p0;
-                    const int lim = q < g.nq ? (g.tri ? min(np, q - p0) : np) : 0;
-                    for (int p = lane; p < pr; p += 32) pb_cp(d + e * LD + p, p < lim ? src + p : V, p < lim);
+                    const int q = q0 + e, lim = (q < g.nq ? (g.tri ? min(np, q - p0) : np) : 0) - lane;
+#pragma unroll
+                    for (int i = 0; i < FT / 4; i++)
+                        if (32 * i < pr) pb_cp(d + 256 * i, 32 * i < lim ? src + 32 * i : V, 32 * i < lim);
+                    src += g.tri ? q : g.np;
+                    d += LD * 8;
                 }
             }
             asm volatile("cp.async.commit_group;" ::: "memory");
         };
 #pragma unroll
         for (int i = 0; i < PST - 1; i++) issue(s0 + i);
+        // r of the strip's rows q and the old outputs of its q product, a strip
+        // ahead like the copies
+        double bq[2], old[2], bqn[2], oldn[2];
+        auto fetch = [&](int s, double (&b)[2], double (&o)[2]) {
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                const int q = 8 * s + 4 * i + lo;
+                b[i] = dop && cl.rq >= 0 && q < g.nq ? __ldg(rq + cl.rq + q) : 0.0;
+                o[i] = doq && cl.oq[i] >= 0 && 8 * s + hi < g.nq ? oq[cl.oq[i] + (8 * s + hi) * os] : 0.0;
+            }
+        };
+        fetch(s0, bq, old);
         for (int s = s0; s < s1; s++) {
             issue(s + PST - 1);
             const int q0 = 8 * s, pr = rows(s);
-            double bq[2], old[2];
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int q = q0 + 4 * i + lo;
-                bq[i] = dop && cl.rq >= 0 && q < g.nq ? __ldg(rq + cl.rq + q) : 0.0;
-                old[i] = doq && cl.oq[i] >= 0 && q0 + hi < g.nq ? oq[cl.oq[i] + (q0 + hi) * os] : 0.0;
-            }
+            fetch(s + 1, bqn, oldn);
             asm volatile("cp.async.wait_group %0;" ::"n"(PST - 1) : "memory");
             __syncwarp();
             const double *d = ring + (s % PST) * pb_strip<FT>();
@@ -128,6 +142,11 @@ __device__ void pb_block(const PairGroup &g, const double *__restrict__ V, const
 #pragma unroll
                 for (int i = 0; i < 2; i++)
                     if (cl.oq[i] >= 0 && q0 + hi < g.nq) oq[cl.oq[i] + (q0 + hi) * os] = old[i] + aq * (c0[i] + c1[i]);
+            }
+#pragma unroll
+            for (int i = 0; i < 2; i++) {
+                bq[i] = bqn[i];
+                old[i] = oldn[i];
             }
             __syncwarp();  // the strip's slot is copied to again
         }
@@ -152,7 +171,7 @@ __device__ void pb_block(const PairGroup &g, const double *__restrict__ V, const
 // W(em,bj): a warp per (block, b, m, column group); the column groups of one
 // block are neighbours, so the list is read from memory once
 template <int FT>
-__global__ void __launch_bounds__(PW * 32) k_pair_wmbej(const PairGroup *__restrict__ groups, int ngroups, i64 items,
+__global__ void __launch_bounds__(PW * 32, 3) k_pair_wmbej(const PairGroup *__restrict__ groups, int ngroups, i64 items,
                                                         int ncg, const double *__restrict__ V,
                                                         const double *__restrict__ r, double *__restrict__ W, double f,
                                                         int nb, i64 rb, i64 wb) {
@@ -186,7 +205,7 @@ __global__ void __launch_bounds__(PW * 32) k_pair_wmbej(const PairGroup *__restr
 // each warp sums its columns in shared memory, then the warps' sums are added
 // in order
 template <int FT>
-__global__ void __launch_bounds__(PW * 32) k_pair_fae(const PairGroup *__restrict__ groups,
+__global__ void __launch_bounds__(PW * 32, 3) k_pair_fae(const PairGroup *__restrict__ groups,
                                                       const int *__restrict__ glist, const int *__restrict__ rowirr,
                                                       const double *__restrict__ V, const double *__restrict__ r,
                                                       double *__restrict__ F, double f, int c0, int nb, i64 rb, i64 fb,
