@@ -514,7 +514,15 @@ int launch_tiles(const ContractPlan *p, const double *A, const double *B, double
     const int bm = TILE_BM[p->cfg], bn = TILE_BN[p->cfg];
     double *part = nullptr;
     ScratchScope scope;
-    if (p->nparts > 0) CPSD_TRY(scratch(p->nparts * bm * bn, &part));
+    if (p->nparts > 0) {
+        const int rc = scratch(p->nparts * bm * bn, &part);
+        // a caller's workspace may hold no more than the fixed rule asks for
+        // (K parts of 256 and more): the same contraction with those tiles
+        const ContractPlan *q = nullptr;
+        if (rc != CPSD_OK && arena().external && plan_fixed(p, &q) == CPSD_OK && q->nparts < p->nparts)
+            return launch_tiles(q, A, B, C, alpha);
+        CPSD_TRY(rc);
+    }
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (timing().on) {
         CPSD_TRY(timing_event(&e0));

@@ -71,3 +71,26 @@ def test_tiles_match_torch(a, b, i, j, e, f, nirrep):
     ref = (d3 + 0.5 * torch.einsum("aebf,eifj->aibj", d1, d2))[tuple(ix.T)]
     K = e * f
     assert float((v3 - ref).abs().max()) < 4 * K * 2.3e-16 * np.sqrt(K) + 1e-14
+
+
+def test_small_workspace_keeps_the_fixed_tiles():
+    """A caller's workspace too small for the chosen K parts still serves a contraction that the fixed rule (parts of
+    256 and more) does without partial tiles."""
+    n, k = 40, 176
+    api.init(1, xor_dirprd(1))
+    api.use_torch_stream()
+    P = {"a": pops(n, 1), "b": pops(n, 1), "e": pops(k, 1), "z": pops(1, 1)}
+    g = torch.Generator(device="cuda").manual_seed(3)
+    A, B = (torch.randn(n * k, dtype=torch.float64, device="cuda", generator=g) for _ in range(2))
+    C = torch.zeros(n * n, dtype=torch.float64, device="cuda")
+    ws = torch.empty(256, dtype=torch.float64, device="cuda")
+    z = P["z"]
+    args = (A, ([P["a"], P["e"], z, z], (1, 1), 1), "ae..", B, ([P["e"], P["b"], z, z], (1, 1), 1), "eb..", C,
+            ([P["a"], P["b"], z, z], (1, 1), 1), "ab..", 1.0, 0.0)
+    api.check(api.lib().cpsd_set_workspace(api.dptr(ws), api.ctypes.c_size_t(ws.numel() * 8)), "workspace")
+    try:
+        api.vv2v_dpd_444(*args)
+    finally:
+        api.check(api.lib().cpsd_set_workspace(None, api.ctypes.c_size_t(0)), "workspace")
+    ref = (B.view(n, k) @ A.view(k, n)).reshape(-1)  # column-major storage
+    assert float((C - ref).abs().max()) < 4 * k * 2.3e-16 * np.sqrt(k)
