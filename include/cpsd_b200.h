@@ -480,7 +480,7 @@ int cpsd_pipeline(const cpsd_system *s, const cpsd_integrals *I, const cpsd_para
 int cpsd_set_phase_overlap(int on);
 /* Empirical tile-shape choice for the FP64 tile kernel (off by default):
  * with it on, the first launch of each contraction plan runs its tile shapes
- * (128x64, 128x32, 64x128, 64x64, 128x16) on a scratch copy of the output,
+ * (128x64, 128x32, 64x128, 64x64) on a scratch copy of the output,
  * times them with CUDA events and keeps the fastest (the cost model's shape
  * unless another is 3 % faster) for every later launch of that plan.  The
  * sums of different shapes differ in rounding, and the choice can differ

@@ -122,7 +122,7 @@ def mixed_error(reset=True):
 def contract_records(maxrec=16384):
     """Per-launch records of the contraction timing buffer (timing must
     have been on, see contract_timing): milliseconds, useful flops, kind
-    (0-4 FP64 tile shapes, 10/11 digit slicing, 12 digit GEMM, 20/21 narrow,
+    (0-3 FP64 tile shapes, 10/11 digit slicing, 12 digit GEMM, 20/21 narrow,
     22 short-K, 23 row-dot and packed pair,
     30/31 Davidson, 32 solver, 40 pair transform) and size triple."""
     ms, fl = np.zeros(maxrec), np.zeros(maxrec)

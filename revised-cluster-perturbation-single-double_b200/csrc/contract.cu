@@ -147,7 +147,6 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
         // one contracted unit: offsets in a constant step, no table
         const bool afast = sg.aMfast, bfast = sg.bKfast, lin = sg.nk == 1;
         const i64 ksa = sg.kSA[0], ksb = sg.kSB[0];
-        const int kend = (int)(ke - kb);
         auto put_a = [&](int buf, int k, int m, i64 om, bool in, i64 ok) {
             stage_cp(&As[buf][k][m], in ? A + om + ok : A, in);
         };
@@ -156,40 +155,42 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
         };
         auto issue = [&](int s) {
             if (s < nst) {
-                const int buf = s % NST, k0 = s * BK;
+                const int buf = s % NST;
+                const i64 k0 = kb + (i64)s * BK;
+                const int left = (int)(ke - k0 < BK ? ke - k0 : BK);  // indices of this stage
                 if (afast) {  // a thread keeps its row (BM divides NT)
                     const int m = tid % BM;
                     const i64 om = offM[m];
 #pragma unroll
                     for (int i = 0; i < LA; i++) {
                         const int k = tid / BM + i * (NT / BM);
-                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksa : offKA[buf][k]);
+                        put_a(buf, k, m, om, om >= 0 && k < left, lin ? (k0 + k) * ksa : offKA[buf][k]);
                     }
                 } else {  // a thread keeps its contracted index
                     const int k = tid % BK;
-                    const i64 ok = lin ? (kb + k0 + k) * ksa : offKA[buf][k];
+                    const i64 ok = lin ? (k0 + k) * ksa : offKA[buf][k];
 #pragma unroll
                     for (int i = 0; i < LA; i++) {
                         const int m = tid / BK + i * (NT / BK);
                         const i64 om = offM[m];
-                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, ok);
+                        put_a(buf, k, m, om, om >= 0 && k < left, ok);
                     }
                 }
                 if (bfast) {
                     const int k = tid % BK;
-                    const i64 ok = lin ? (kb + k0 + k) * ksb : offKB[buf][k];
+                    const i64 ok = lin ? (k0 + k) * ksb : offKB[buf][k];
 #pragma unroll
                     for (int i = 0; i < LB; i++) {
                         const int n = tid / BK + i * (NT / BK);
                         const i64 on = offN[n];
-                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, ok);
+                        put_b(buf, k, n, on, on >= 0 && k < left, ok);
                     }
                 } else {
 #pragma unroll
                     for (int i = 0; i < LB; i++) {
                         const int e = tid + i * NT, n = e % BN, k = e / BN;
                         const i64 on = offN[n];
-                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksb : offKB[buf][k]);
+                        put_b(buf, k, n, on, on >= 0 && k < left, lin ? (k0 + k) * ksb : offKB[buf][k]);
                     }
                 }
             }
@@ -417,7 +418,7 @@ int tune_plan(const ContractPlan *p, const double *A, const double *B, const Con
     CPSD_TRY(cuda_check(cudaEventCreate(&e1), "event"));
     float best_ms = 1e30f;
     int rc = CPSD_OK;
-    for (int c = 0; c < NTILE && rc == CPSD_OK; c++) {
+    for (int c = 0; c < NTILE - 1 && rc == CPSD_OK; c++) {
         const ContractPlan *q = p;
         if (c != p->cfg) {
             auto v = std::make_unique<ContractPlan>();
@@ -511,7 +512,7 @@ void run_tiles(int cfg, int ntiles, const double *A, const double *B, double *C,
 
 int launch_tiles(const ContractPlan *p, const double *A, const double *B, double *C, double alpha) {
     CPSD_TRY(const_cast<ContractPlan *>(p)->upload());
-    const int bm = TILE_BM[p->cfg], bn = TILE_BN[p->cfg];
+    const int bm = TILE_BM[p->shape()], bn = TILE_BN[p->shape()];
     double *part = nullptr;
     ScratchScope scope;
     if (p->nparts > 0) {
@@ -532,7 +533,7 @@ int launch_tiles(const ContractPlan *p, const double *A, const double *B, double
         CPSD_TRY(cuda_check(cudaEventRecord(e0, stream()), "event record"));
     }
     CPSD_TRY(tile_attrs());
-    run_tiles(p->cfg, p->ntiles, A, B, C, p->d_tasks, p->d_segs, p->d_tiles, alpha, part);
+    run_tiles(p->shape(), p->ntiles, A, B, C, p->d_tasks, p->d_segs, p->d_tiles, alpha, part);
     count_launch();
     ctx().flops += p->flops;
     if (e1) CPSD_TRY(cuda_check(cudaEventRecord(e1, stream()), "event record"));

@@ -116,6 +116,7 @@ void choose_tiles(const std::vector<TaskDev> &tasks, int force_cfg, int *cfg_out
     double best = 1e300;
     for (int c = 0; c < NTILE; c++) {
         if (force_cfg >= 0 && c != force_cfg) continue;
+        if (c == NTILE - 1 && std::any_of(tasks.begin(), tasks.end(), [](const TaskDev &t) { return t.N > 16; })) continue;
         const i64 bm = TILE_BM[c], bn = TILE_BN[c], slots = TILE_CTAS[c] * SMS;
         // time of a K stage of 16 with r CTAs on the SM
         auto stage = [&](i64 r) {
@@ -197,6 +198,8 @@ void finish_plan(ContractPlan *plan, std::vector<TaskDev> tasks, std::vector<Seg
     if (fixed) choose_tiles_fixed(tasks, &cfg, &split);
     else choose_tiles(tasks, force_cfg, &cfg, &split);
     const i64 minpart = fixed ? FIXED_MINPART : MINPART;
+    plan->cols16 = cfg == NTILE - 1;
+    if (plan->cols16) cfg = 1;
     const i64 TBM = TILE_BM[cfg], TBN = TILE_BN[cfg];
     plan->cfg = cfg;
     std::vector<TileDev> tiles;

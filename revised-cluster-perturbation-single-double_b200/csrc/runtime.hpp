@@ -162,7 +162,9 @@ struct TileDev {
     i64 part;            // partial slot (split-K) or -1
 };
 
-// tile shapes of the contraction kernel: BM x BN = 128x64, 128x32, 64x128, 64x64, 128x16
+// tile shapes of the contraction kernel: BM x BN = 128x64, 128x32, 64x128, 64x64;
+// the last one, 128x16, runs the 128x32 tiles of a plan whose outputs have at
+// most 16 columns (cols16)
 constexpr int NTILE = 5;
 extern const int TILE_BM[NTILE];
 extern const int TILE_BN[NTILE];
@@ -170,6 +172,8 @@ extern const int TILE_BN[NTILE];
 struct ContractPlan {
     bool empty = true;
     int cfg = 0;  // tile shape (index into TILE_BM / TILE_BN)
+    bool cols16 = false;  // 128x32 tiles run by the 128x16 kernel
+    int shape() const { return cols16 ? NTILE - 1 : cfg; }
     int ntasks = 0, nsegs = 0, ntiles = 0;
     i64 nparts = 0;      // split-K partial tiles
     // host tables (kept for introspection) and their device copies,
@@ -256,7 +260,7 @@ int launch_contract(const ContractPlan *p, const double *A, const double *B, dou
 int launch_contract_noalloc(const ContractPlan *p, const double *A, const double *B, double *C, double alpha);
 size_t contract_noalloc_bytes(const ContractPlan *p);
 // CUDA-event record of one more launch in the timing buffer (when timing is
-// on): kind 0-4 DMMA tile shapes, 10 / 11 digit slicing of A / B, 12 digit
+// on): kind 0-3 DMMA tile shapes, 10 / 11 digit slicing of A / B, 12 digit
 // GEMM, 20 / 21 narrow-output kernels (rows / K), 22 short-K kernel (tasks,
 // tiles, output elements), 23 row-dot kernel (tasks, warps, output
 // elements), 30 / 31 Davidson step /
