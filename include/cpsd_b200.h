@@ -350,6 +350,10 @@ int cpsd_debug_ozaki_plan(const cpsd_opt *v1, const char *t1, const cpsd_opt *v2
  * wi[k] > 0: real and imaginary parts; unit norm, largest component real);
  * *sweeps = QR sweeps or -1 when the iteration did not converge */
 int cpsd_debug_geev(const double *A_host, int64_t n, double *wr, double *wi, double *V_host, int64_t *sweeps);
+/* its symmetric eigen-solve (cyclic Jacobi): eigenvalues w and row-major V
+ * whose column k is the eigenvector of w[k], of the sign that the order of the
+ * rotations gives */
+int cpsd_debug_syev(const double *A_host, int64_t n, double *w, double *V_host);
 int cpsd_debug_pairmap_plan(const cpsd_opt *in, int64_t op0, int64_t op1, int64_t tgt0, int64_t tgt1,
                             const void **blocks, int64_t *nblocks, const void **idx, const void **sgn,
                             int64_t *nidx, int64_t *lterms, int64_t *rterms);

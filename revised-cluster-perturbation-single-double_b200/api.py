@@ -176,6 +176,17 @@ def geev(A):
     return wr, wi, V, sw.value
 
 
+def syev(A):
+    """The Davidson step's symmetric eigen-solve on a host matrix (n <= 32):
+    (w, V), column k of V the eigenvector of w[k]."""
+    A = np.ascontiguousarray(A, dtype=np.float64)
+    n = A.shape[0]
+    w, V = np.zeros(n), np.zeros((n, n))
+    check(lib().cpsd_debug_syev(A.ctypes.data_as(ctypes.c_void_p), I64(n), w.ctypes.data_as(ctypes.c_void_p),
+                                V.ctypes.data_as(ctypes.c_void_p)), "cpsd_debug_syev")
+    return w, V
+
+
 def opt(pops, iops, sym, t):
     o = Opt()
     check(lib().cpsd_opt_init(ctypes.byref(o), arr8(pops[0]), arr8(pops[1]), arr8(pops[2]), arr8(pops[3]),

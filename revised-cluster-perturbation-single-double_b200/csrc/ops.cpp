@@ -1316,6 +1316,19 @@ int cpsd_debug_geev(const double *A_host, int64_t n, double *wr, double *wi, dou
     return CPSD_OK;
 }
 
+int cpsd_debug_syev(const double *A_host, int64_t n, double *w, double *V_host) {
+    if (n < 1 || n > DAV_MAXD) return set_error(CPSD_EARG, "n must be 1..32");
+    ScratchScope sc;
+    double *dA, *dw, *dV;
+    CPSD_TRY(scratch(n * n, &dA));
+    CPSD_TRY(scratch(n, &dw));
+    CPSD_TRY(scratch(n * n, &dV));
+    CPSD_TRY(cuda_check(cudaMemcpyAsync(dA, A_host, sizeof(double) * n * n, cudaMemcpyHostToDevice, stream()), "syev A"));
+    CPSD_TRY(syev_probe(dA, (int)n, dw, dV));
+    CPSD_TRY(read_back(w, dw, sizeof(double) * n));
+    return read_back(V_host, dV, sizeof(double) * n * n);
+}
+
 int64_t cpsd_irpdso(int64_t sym, const int64_t *popp, const int64_t *popq, int64_t ioppq) {
     return irpdso(sym, popp, popq, ioppq);
 }

@@ -152,10 +152,34 @@ __device__ double warp_dot(const double *x, const double *y, int n) {
 
 constexpr int GL = DAV_MAXD + 1;
 
-// Cyclic Jacobi on the symmetric n x n matrix in S (ld GL, zero outside
-// n x n) by the whole block; the eigenvalues end on the diagonal of S, the
-// eigenvectors in the columns of V (ld GL).  S2 and V2 are scratch of the
-// same size.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an element
+// Index that round robin pairing r (0 <= r < m - 1) of m = 2, 4, .. indices has
+// at place i: places 2k and 2k + 1 are a pair, {m - 1, r} for k = 0 and {r - k,
+// r + k} modulo m - 1 for the others
+__device__ __forceinline__ int jacobi_at(int i, int m, int r) {
+    const int k = i >> 1;
+    if (i & 1) return r + k < m - 1 ? r + k : r + k - (m - 1);
+    return k == 0 ? m - 1 : r - k >= 0 ? r - k : r - k + m - 1;
+}
+
+// The symmetric n x n matrix a(i, j) into S (ld GL) in the places of the first
+// pairing of m = n rounded up to even, zero where an index is n: the padding of
+// an odd n, which sits at place 0 throughout
+template <class F>
+__device__ void jacobi_place(double *S, int n, F a) {
+    const int m = (n + 1) & ~1;
+    for (int e = threadIdx.x; e < DAV_MAXD * DAV_MAXD; e += DT) {
+        const int p = e / DAV_MAXD, q = e % DAV_MAXD;
+        const int i = p < m ? jacobi_at(p, m, 0) : n, j = q < m ? jacobi_at(q, m, 0) : n;
+        S[p * GL + q] = i < n && j < n ? a(i, j) : 0.0;
+    }
+    __syncthreads();
+}
+
+// Cyclic Jacobi by the whole block on the symmetric n x n matrix that
+// jacobi_place put into S: w receives the eigenvalues, the columns of V (ld
+// GL) the eigenvectors; S2 and V2 are scratch of the same size.  The order of
+// the rotations is part of the result, as it decides the sign of every
+// eigenvector.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an element
 // with a_pq^2 <= 1e-34 |a_pp a_qq| is negligible and set to zero.  The
 // n(n-1)/2 rotations of a sweep run as n-1 rounds of n/2 disjoint rotations
 // (round-robin pairing, n padded to even), each round one parallel update of
@@ -174,14 +198,14 @@ constexpr int GL = DAV_MAXD + 1;
 // of the next round's pairing, in the other of two buffers: every address of
 // a thread is the same in all rounds.  (Indexing the pairs anew took 1250
 // cycles a round; roots, divisions and the index arithmetic 2000.)
-__device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n) {
+__device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n, double *w) {
     __shared__ double cs[DAV_MAXD / 2], sn[DAV_MAXD / 2], tn[DAV_MAXD / 2];
     __shared__ int rotate;  // last round that saw an element above the threshold
     const int tid = threadIdx.x;
     const int m = (n + 1) & ~1, half = m / 2;
     for (int e = tid; e < DAV_MAXD * DAV_MAXD; e += DT) {
         const int i = e / DAV_MAXD, j = e % DAV_MAXD;
-        V[i * GL + j] = (i == j && i < m) ? 1.0 : 0.0;
+        V[i * GL + j] = (j < m && i == jacobi_at(j, m, 0)) ? 1.0 : 0.0;
         V2[i * GL + j] = 0.0;
     }
     if (tid == 0) rotate = 0;
@@ -235,6 +259,7 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
     }
     const bool dia = on_s && k0 == l0;
     double *A = S, *B = S2, *E = V, *F = V2;
+    int r = 0;  // pairing of the round
     __syncthreads();
     for (int round = 1; round <= 50 * (m - 1); round++) {
         // does any element of the matrix still call for a rotation?
@@ -270,7 +295,8 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
             }
             const double h = rsqrt(h2), u = fma(0.5 * fabs(d), h, 0.5), ru = rsqrt(u);
             double s = 0.5 * fabs(b) * h * ru;
-            if (d != 0.0 && ((d > 0.0) != (b > 0.0))) s = -s;
+            // equal diagonal elements: t = 1 from the lower to the higher index
+            if (d == 0.0 ? jacobi_at(2 * tid, m, r) > jacobi_at(2 * tid + 1, m, r) : (d > 0.0) != (b > 0.0)) s = -s;
             cs[tid] = keep ? 1.0 : u * ru;
             sn[tid] = keep ? 0.0 : s;
             tn[tid] = keep ? 0.0 : s * ru;  // s / c
@@ -310,26 +336,24 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
         x = E;
         E = F;
         F = x;
+        r = r + 1 < m - 1 ? r + 1 : 0;
         __syncthreads();
     }
-    // the padding of an odd n sits at place p: it goes last
-    if (A != S)
-        for (int e = tid; e < m * m; e += DT) {
-            const int i = e / m, j = e % m;
-            S[i * GL + j] = A[i * GL + j];
-            V[i * GL + j] = E[i * GL + j];
-        }
+    // back from the places of the last pairing, two elements of V a thread
+    if (tid < m && jacobi_at(tid, m, r) < n) w[jacobi_at(tid, m, r)] = A[tid * (GL + 1)];
+    double v[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int e = tid + u * DT;
+        v[u] = E[e / DAV_MAXD * GL + e % DAV_MAXD];
+    }
     __syncthreads();
-    if (m > n) {
-        __shared__ int pad;
-        if (tid < m && V[n * GL + tid] == 1.0) pad = tid;
-        __syncthreads();
-        if (pad != n) {
-            if (tid == 0) S[pad * (GL + 1)] = S[n * (GL + 1)];
-            if (tid < m) V[tid * GL + pad] = V[tid * GL + n];
-        }
-        __syncthreads();
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        const int e = tid + u * DT, j = e % DAV_MAXD;
+        if (j < m) V[e / DAV_MAXD * GL + jacobi_at(j, m, r)] = v[u];
     }
+    __syncthreads();
 }
 
 // ------------------------------------------------ general real eigenproblem
@@ -944,13 +968,8 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int
         }
         __syncthreads();
         if (!general) {
-            for (int e = tid; e < DAV_MAXD * DAV_MAXD; e += DT) {
-                int i = e / DAV_MAXD, j = e % DAV_MAXD;
-                S[i * GL + j] = (i < dimIter && j < dimIter) ? 0.5 * (s.Abar[i + j * D] + s.Abar[j + i * D]) : 0.0;
-            }
-            __syncthreads();
-            block_jacobi(S, V, X, sm.tot, dimIter);
-            if (tid < dimIter) vR[tid] = S[tid * GL + tid];
+            jacobi_place(S, dimIter, [&](int i, int j) { return 0.5 * (s.Abar[i + j * D] + s.Abar[j + i * D]); });
+            block_jacobi(S, V, X, sm.tot, dimIter, vR);
         } else {
             for (int e = tid; e < dimIter * dimIter; e += DT) {
                 const int i = e / dimIter, j = e % dimIter;
@@ -1700,7 +1719,23 @@ __global__ void __launch_bounds__(32) k_geev_probe(const double *A, int n, doubl
     if (threadIdx.x == 0) *sweeps = sw;
 }
 
+// the symmetric eigen-solve of the Davidson step on one given matrix
+__global__ void __launch_bounds__(DT) k_syev_probe(const double *A, int n, double *wr, double *V) {
+    __shared__ double S[DAV_MAXD * GL], S2[DAV_MAXD * GL], U[DAV_MAXD * GL], U2[DAV_MAXD * GL], w[DAV_MAXD];
+    jacobi_place(S, n, [&](int i, int j) { return A[i * n + j]; });
+    block_jacobi(S, U, S2, U2, n, w);
+    if ((int)threadIdx.x < n) wr[threadIdx.x] = w[threadIdx.x];
+    for (int e = threadIdx.x; e < n * n; e += DT) V[e] = U[(e / n) * GL + e % n];
+}
+
 }  // namespace
+
+int syev_probe(const double *A_dev, int n, double *w, double *V) {
+    if (n < 1 || n > DAV_MAXD) return set_error(CPSD_EARG, "syev: n must be 1..32");
+    k_syev_probe<<<1, DT, 0, stream()>>>(A_dev, n, w, V);
+    count_launch();
+    return cuda_check(cudaGetLastError(), "k_syev_probe");
+}
 
 int geev_probe(const double *A_dev, int n, double *wr, double *wi, double *V, int *sweeps) {
     if (n < 1 || n > DAV_MAXD) return set_error(CPSD_EARG, "geev: n must be 1..32");

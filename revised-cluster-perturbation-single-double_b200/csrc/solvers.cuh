@@ -45,6 +45,9 @@ int dav_final_launch(DavState *st, const DavBuffers &b);     // eigen test resid
 // matrix: eigenvalues wr / wi, eigenvectors V (row-major, dgeev's columns),
 // QR sweeps (-1: no convergence); all device pointers
 int geev_probe(const double *A_dev, int n, double *wr, double *wi, double *V, int *sweeps);
+// the same of its symmetric eigen-solve: eigenvalues w, column k of V the
+// eigenvector of w[k]
+int syev_probe(const double *A_dev, int n, double *w, double *V);
 
 constexpr int DIIS_MAXDIM = 16;
 struct DiisState {
