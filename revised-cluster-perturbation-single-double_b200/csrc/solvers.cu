@@ -189,8 +189,9 @@ __device__ void jacobi_place(double *S, int n, F a) {
 // d / b, d = a_qq - a_pp, b = 2 a_pq, by its half angle:
 //   h = 1 / sqrt(d^2 + b^2),  u = (1 + |d| h) / 2,  r = 1 / sqrt(u),
 //   c = u r,  s = sgn(d b) |b| h r / 2,
-// two reciprocal roots after one another and no division; a pair whose
-// d^2 + b^2 leaves the normal range is scaled first.
+// two reciprocal roots after one another and no division, and one correction
+// of c^2 + s^2 to 1; a pair whose d^2 + b^2 leaves the normal range is scaled
+// first.
 //
 // Latency bounds it: about 80 rounds at n = 20, each a chain of the rotation
 // parameters, a barrier, one 2 x 2 update and a barrier.  So pair k always
@@ -294,10 +295,16 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
                 h2 = fma(d, d, b * b);
             }
             const double h = rsqrt(h2), u = fma(0.5 * fabs(d), h, 0.5), ru = rsqrt(u);
-            double s = 0.5 * fabs(b) * h * ru;
+            double c = u * ru, s = 0.5 * fabs(b) * h * ru;
+            // c and s hold the rounding of h apart from one another: scaled to
+            // c^2 + s^2 = 1 (the defect itself, not 1 less half of it, which
+            // would round one way only)
+            const double z = fma(-s, s, fma(-c, c, 1.0));
+            c = fma(0.5 * c, z, c);
+            s = fma(0.5 * s, z, s);
             // equal diagonal elements: t = 1 from the lower to the higher index
             if (d == 0.0 ? jacobi_at(2 * tid, m, r) > jacobi_at(2 * tid + 1, m, r) : (d > 0.0) != (b > 0.0)) s = -s;
-            cs[tid] = keep ? 1.0 : u * ru;
+            cs[tid] = keep ? 1.0 : c;
             sn[tid] = keep ? 0.0 : s;
             tn[tid] = keep ? 0.0 : s * ru;  // s / c
         }
