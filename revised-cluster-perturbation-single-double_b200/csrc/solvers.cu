@@ -1450,12 +1450,14 @@ __global__ void __launch_bounds__(DT) k_dav_final(DavState *st, DavBuffers b, co
 // ------------------------------------------------------------------- DIIS
 // LINPACK dgefa / dgesl (as MINV, src/libsrint/minv.f, calls them) by one
 // warp on a matrix in shared memory (n <= 32): lane i owns row i.  Pivot =
-// first row of largest magnitude; every element sees the same operations in
+// first row of largest magnitude, NaN counting as the largest (compared as it
+// is, it would leave the lanes with different rows and some with none); every element sees the same operations in
 // the same order as the sequential LINPACK loops.
 __device__ void warp_dgefa(double *a, int lda, int n, int *ipvt) {
     const int i = threadIdx.x & 31;
     for (int k = 0; k < n - 1; k++) {
         double m = (i >= k && i < n) ? fabs(a[i + k * lda]) : -1.0;
+        if (!(m >= -1.0)) m = HUGE_VAL;
         int l = (i >= k && i < n) ? i : 0x7fffffff;
         for (int o = 16; o > 0; o >>= 1) {
             double om = __shfl_xor_sync(0xffffffffu, m, o);

@@ -1,5 +1,6 @@
-"""NaN and infinities in the symmetric Ritz problem: the eigen-solve and the SF-CIS program end without an error, with
-NaN values and without a write outside their buffers, for even and odd subspaces (an odd one is padded by one place)."""
+"""NaN and infinities in the solvers.  Symmetric Ritz problem: the eigen-solve and the SF-CIS program end without an error,
+with NaN values and without a write outside their buffers, for even and odd subspaces (an odd one is padded by one
+place).  DIIS: the same of the loop whose pivots are NaN."""
 import numpy as np
 import pytest
 
@@ -36,3 +37,16 @@ def test_cis_takes_nan(roots):
                      run_opts=dict(lowest=1))
     again, _, _ = api.cis_run(s, api.make_system(s), api.DeviceIntegrals(s), api.make_params(s))
     assert np.array_equal(good, again)
+
+
+def test_diis_takes_nan():
+    s = synth.System(nmo=24, nocc_a=5, nocc_b=3, nirrep=2, seed=6, roots=1)
+    api.use_torch_stream()
+    good = api.ground(s, api.make_system(s), api.DeviceIntegrals(s), api.make_params(s))
+    for x in s.ints.values():
+        x[:] = np.nan
+    bad = api.ground(s, api.make_system(s), api.DeviceIntegrals(s), api.make_params(s))
+    assert np.isnan(bad["E3"]) and torch.isnan(bad["T1_2"]).any()
+    s = synth.System(nmo=24, nocc_a=5, nocc_b=3, nirrep=2, seed=6, roots=1)
+    again = api.ground(s, api.make_system(s), api.DeviceIntegrals(s), api.make_params(s))
+    assert good["E3"] == again["E3"] and torch.equal(good["T1_2"], again["T1_2"])
