@@ -84,15 +84,6 @@ __global__ void k_eri_adjoint(const i64 *__restrict__ blk, int nblocks, i64 n, c
     }
 }
 
-template <class T>
-int upload_vec(const std::vector<T> &v, T **d) {
-    *d = nullptr;
-    if (v.empty()) return CPSD_OK;
-    CPSD_TRY(cuda_check(cudaMalloc(d, sizeof(T) * v.size()), "cudaMalloc(eri plan)"));
-    return cuda_check(cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()),
-                      "upload eri plan");
-}
-
 // the six lists: slot kinds, iops and the slot -> <PQ||RS> map
 // (allocate_mem.f90:14-44; iabj(b,i,a,j) = <ia||bj>)
 struct ListKind {
@@ -138,9 +129,9 @@ int plan_eri_list(const Sys &S, int which, const EriListPlan **out) {
     }
     plan->n = off;
     plan->nblocks = (int)(blk.size() / 5);
-    CPSD_TRY(upload_vec(blk, &plan->d_blk));
-    CPSD_TRY(upload_vec(lp, &plan->d_lp));
-    CPSD_TRY(upload_vec(rp, &plan->d_rp));
+    CPSD_TRY(upload_table(blk, &plan->d_blk, "eri plan"));
+    CPSD_TRY(upload_table(lp, &plan->d_lp, "eri plan"));
+    CPSD_TRY(upload_table(rp, &plan->d_rp, "eri plan"));
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "eri plan upload"));
     *out = plan.get();
     cache[key] = std::move(plan);

@@ -291,23 +291,14 @@ __global__ void __launch_bounds__(NW * 32) k_narrow_reduce(const TaskDev *__rest
         C[tk.baseC + v.crow(rd.r0 + i) + v.ccol(rd.c0 + c)] += alpha * s;
 }
 
-template <class T>
-int upload_vec(const std::vector<T> &v, T **d) {
-    *d = nullptr;
-    if (v.empty()) return CPSD_OK;
-    CPSD_TRY(cuda_check(cudaMalloc(d, sizeof(T) * v.size()), "cudaMalloc(narrow plan)"));
-    return cuda_check(cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()),
-                      "upload narrow plan");
-}
-
 }  // namespace
 
 int NarrowPlan::upload() {
     if (uploaded.load(std::memory_order_acquire)) return CPSD_OK;
     std::lock_guard<std::mutex> lock(upload_mutex());
     if (uploaded.load(std::memory_order_relaxed)) return CPSD_OK;
-    CPSD_TRY(upload_vec(items, &d_items));
-    CPSD_TRY(upload_vec(reds, &d_reds));
+    CPSD_TRY(upload_table(items, &d_items, "narrow plan"));
+    CPSD_TRY(upload_table(reds, &d_reds, "narrow plan"));
     // the tables may next be read by kernels on another thread's stream
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "plan upload"));
     uploaded.store(true, std::memory_order_release);

@@ -478,7 +478,7 @@ namespace {
 
 int oz_error_word(int **err) {
     if (!ctx().oz_err) {
-        CPSD_TRY(cuda_check(cudaMalloc(&ctx().oz_err, sizeof(int)), "cudaMalloc(error word)"));
+        CPSD_TRY(device_alloc(sizeof(int), (void **)&ctx().oz_err, "error word"));
         CPSD_TRY(cuda_check(cudaMemsetAsync(ctx().oz_err, 0, sizeof(int), stream()), "clear error word"));
     }
     *err = ctx().oz_err;

@@ -41,13 +41,7 @@ uint64_t fnv(uint64_t h, const void *p, size_t n) {
 
 template <class T>
 int upload_vec(const std::vector<T> &v, const T **d) {
-    *d = nullptr;
-    if (v.empty()) return CPSD_OK;
-    T *p = nullptr;
-    CPSD_TRY(cuda_check(cudaMalloc(&p, sizeof(T) * v.size()), "cudaMalloc(digit plan)"));
-    *d = p;
-    return cuda_check(cudaMemcpyAsync(p, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()),
-                      "upload digit plan");
+    return upload_table(v, const_cast<T **>(d), "digit plan");
 }
 
 i64 roundup(i64 x, i64 m) { return (x + m - 1) / m * m; }
@@ -65,8 +59,7 @@ int OzPlan::upload() {
     CPSD_TRY(upload_vec(mcombo, &dev.mcombo));
     CPSD_TRY(upload_vec(ncombo, &dev.ncombo));
     dev.ntiles = (int)tiles.size();
-    const int *kc = nullptr;
-    CPSD_TRY(upload_vec(kcombo, &kc));
+    CPSD_TRY(upload_vec(kcombo, &adev.kcombo));
     CPSD_TRY(upload_vec(ajobs, &adev.jobs));
     CPSD_TRY(upload_vec(aroff, &adev.roff));
     CPSD_TRY(upload_vec(akoff, &adev.koff));
@@ -76,13 +69,12 @@ int OzPlan::upload() {
     bdev.kt_max = kt_max;
     bdev.nexpo = neb;
     adev.rcombo = dev.mcombo;
-    adev.kcombo = kc;
     CPSD_TRY(upload_vec(bjobs, &bdev.jobs));
     CPSD_TRY(upload_vec(broff, &bdev.roff));
     CPSD_TRY(upload_vec(bkoff, &bdev.koff));
     bdev.njobs = (int)bjobs.size();
     bdev.rcombo = dev.ncombo;
-    bdev.kcombo = kc;
+    bdev.kcombo = adev.kcombo;
     CPSD_TRY(upload_vec(astage, &adev.stage));
     CPSD_TRY(upload_vec(bstage, &bdev.stage));
     // the tables may next be read by kernels on another thread's stream

@@ -279,15 +279,6 @@ int cached(std::map<std::string, std::unique_ptr<PairBlkPlan>> &cache, std::mute
     return CPSD_OK;
 }
 
-template <class T>
-int put(const std::vector<T> &v, T **d) {
-    *d = nullptr;
-    if (v.empty()) return CPSD_OK;
-    CPSD_TRY(cuda_check(cudaMalloc(d, sizeof(T) * v.size()), "cudaMalloc(pair plan)"));
-    return cuda_check(cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()),
-                      "upload pair plan");
-}
-
 template <int FT>
 int pb_attr(const void *k, size_t smem, std::atomic<bool> &done) {
     if (done.load(std::memory_order_acquire)) return CPSD_OK;
@@ -334,9 +325,9 @@ int PairBlkPlan::upload() {
     if (uploaded.load(std::memory_order_acquire)) return CPSD_OK;
     std::lock_guard<std::mutex> lock(upload_mutex());
     if (uploaded.load(std::memory_order_relaxed)) return CPSD_OK;
-    CPSD_TRY(put(groups, &d_groups));
-    CPSD_TRY(put(glist, &d_glist));
-    CPSD_TRY(put(rowirr, &d_rowirr));
+    CPSD_TRY(upload_table(groups, &d_groups, "pair plan"));
+    CPSD_TRY(upload_table(glist, &d_glist, "pair plan"));
+    CPSD_TRY(upload_table(rowirr, &d_rowirr, "pair plan"));
     // the tables may next be read by kernels on another thread's stream
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "plan upload"));
     uploaded.store(true, std::memory_order_release);

@@ -24,18 +24,6 @@ namespace cpsd {
 
 namespace {
 
-template <class T>
-int upload(const std::vector<T> &v, T **d) {
-    *d = nullptr;
-    if (v.empty()) return CPSD_OK;
-    CPSD_TRY(cuda_check(cudaMalloc(d, sizeof(T) * v.size()), "cudaMalloc(plan)"));
-    // on the library stream: the kernels that read the tables are queued
-    // behind the copy on the same stream (a legacy-stream cudaMemcpy from
-    // pageable memory may still be in flight when it returns)
-    return cuda_check(cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()),
-                      "upload plan");
-}
-
 bool is_zorb(const i64 *p) {
     if (p[0] != 1) return false;
     for (int i = 1; i < 8; i++)
@@ -58,10 +46,10 @@ int ContractPlan::upload() {
     if (uploaded.load(std::memory_order_acquire)) return CPSD_OK;
     std::lock_guard<std::mutex> lock(upload_mutex());
     if (uploaded.load(std::memory_order_relaxed)) return CPSD_OK;
-    CPSD_TRY(cpsd::upload(h_tasks, &d_tasks));
-    CPSD_TRY(cpsd::upload(h_segs, &d_segs));
-    CPSD_TRY(cpsd::upload(h_tiles, &d_tiles));
-    CPSD_TRY(cpsd::upload(h_reduce, &d_reduce));
+    CPSD_TRY(upload_table(h_tasks, &d_tasks, "plan"));
+    CPSD_TRY(upload_table(h_segs, &d_segs, "plan"));
+    CPSD_TRY(upload_table(h_tiles, &d_tiles, "plan"));
+    CPSD_TRY(upload_table(h_reduce, &d_reduce, "plan"));
     // the tables may next be read by kernels on another thread's stream
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "plan upload"));
     uploaded.store(true, std::memory_order_release);
@@ -71,10 +59,10 @@ int PairMapPlan::upload() {
     if (uploaded.load(std::memory_order_acquire)) return CPSD_OK;
     std::lock_guard<std::mutex> lock(upload_mutex());
     if (uploaded.load(std::memory_order_relaxed)) return CPSD_OK;
-    CPSD_TRY(cpsd::upload(h_blocks, &d_blocks));
-    CPSD_TRY(cpsd::upload(h_idx, &d_idx));
-    CPSD_TRY(cpsd::upload(h_sgn, &d_sgn));
-    if (tiled) CPSD_TRY(cpsd::upload(h_tstart, &d_tstart));
+    CPSD_TRY(upload_table(h_blocks, &d_blocks, "plan"));
+    CPSD_TRY(upload_table(h_idx, &d_idx, "plan"));
+    CPSD_TRY(upload_table(h_sgn, &d_sgn, "plan"));
+    if (tiled) CPSD_TRY(upload_table(h_tstart, &d_tstart, "plan"));
     // the tables may next be read by kernels on another thread's stream
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "plan upload"));
     uploaded.store(true, std::memory_order_release);
@@ -84,9 +72,9 @@ int EnergyPlan::upload() {
     if (uploaded.load(std::memory_order_acquire)) return CPSD_OK;
     std::lock_guard<std::mutex> lock(upload_mutex());
     if (uploaded.load(std::memory_order_relaxed)) return CPSD_OK;
-    CPSD_TRY(cpsd::upload(h_blk, &d_blk));
-    CPSD_TRY(cpsd::upload(h_lidx, &d_lidx));
-    CPSD_TRY(cpsd::upload(h_ridx, &d_ridx));
+    CPSD_TRY(upload_table(h_blk, &d_blk, "plan"));
+    CPSD_TRY(upload_table(h_lidx, &d_lidx, "plan"));
+    CPSD_TRY(upload_table(h_ridx, &d_ridx, "plan"));
     // the tables may next be read by kernels on another thread's stream
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "plan upload"));
     uploaded.store(true, std::memory_order_release);

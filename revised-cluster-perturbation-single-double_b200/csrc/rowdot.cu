@@ -187,24 +187,15 @@ __global__ void __launch_bounds__(RW * 32) k_rowdot(const TaskDev *__restrict__ 
     cp_async_wait<0>();  // no copy outlives the warp
 }
 
-template <class T>
-int upload_vec(const std::vector<T> &v, T **d) {
-    *d = nullptr;
-    if (v.empty()) return CPSD_OK;
-    CPSD_TRY(cuda_check(cudaMalloc(d, sizeof(T) * v.size()), "cudaMalloc(row-dot plan)"));
-    return cuda_check(cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()),
-                      "upload row-dot plan");
-}
-
 }  // namespace
 
 int RowDotPlan::upload() {
     if (uploaded.load(std::memory_order_acquire)) return CPSD_OK;
     std::lock_guard<std::mutex> lock(upload_mutex());
     if (uploaded.load(std::memory_order_relaxed)) return CPSD_OK;
-    CPSD_TRY(upload_vec(items, &d_items));
-    CPSD_TRY(upload_vec(tasks, &d_tasks));
-    CPSD_TRY(upload_vec(segs, &d_segs));
+    CPSD_TRY(upload_table(items, &d_items, "row-dot plan"));
+    CPSD_TRY(upload_table(tasks, &d_tasks, "row-dot plan"));
+    CPSD_TRY(upload_table(segs, &d_segs, "row-dot plan"));
     // the table may next be read by kernels on another thread's stream
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "plan upload"));
     uploaded.store(true, std::memory_order_release);

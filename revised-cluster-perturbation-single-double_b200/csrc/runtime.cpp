@@ -207,4 +207,19 @@ int Arena::alloc(size_t bytes, void **out) {
     return CPSD_OK;
 }
 
+int device_alloc(size_t bytes, void **p, const char *what) {
+    *p = nullptr;
+    const double t0 = mem_trace_on() ? host_ms() : 0.0;
+    cudaError_t e = cudaMalloc(p, bytes);
+    for (int k = 0; k < 3 && e == cudaErrorMemoryAllocation; k++) {
+        cudaGetLastError();
+        if (k == 0) pool_release_idle();
+        else if (k == 1) evict_cached_copies(bytes);
+        else arena().trim();
+        e = cudaMalloc(p, bytes);
+        if (mem_trace_on()) mem_trace("table cudaMalloc after release", bytes, host_ms() - t0, e == cudaSuccess);
+    }
+    return cuda_check(e, what);
+}
+
 }  // namespace cpsd

@@ -131,6 +131,19 @@ size_t pool_idle_bytes();
 // pool (its size in *bytes; nullptr if none): device memory that changes
 // hands without a cudaFree / cudaMalloc
 void *pool_take_idle(size_t min_bytes, size_t max_bytes, size_t *bytes);
+// device memory that stays (plan tables, error words): where the driver has no
+// room, idle pool buffers, then cached copies of constant operands (with 256 MB
+// to spare), then this thread's unused scratch chunks give way
+int device_alloc(size_t bytes, void **p, const char *what);
+// a table to the device, queued on the library stream, as the kernels that read
+// it are (a legacy-stream cudaMemcpy from pageable memory may still be in
+// flight when it returns); a buffer that an earlier, failed upload left is used
+template <class T>
+int upload_table(const std::vector<T> &v, T **d, const char *what) {
+    if (v.empty()) return CPSD_OK;
+    if (!*d) CPSD_TRY(device_alloc(sizeof(T) * v.size(), (void **)d, what));
+    return cuda_check(cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()), what);
+}
 struct ScratchScope {
     Arena::Mark m;
     ScratchScope() : m(arena().mark()) {}

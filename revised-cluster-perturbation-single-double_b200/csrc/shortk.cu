@@ -185,15 +185,6 @@ constexpr size_t shortk_smem(int kmax) {
     return sizeof(double) * (size_t)kmax * (size_t)((2048 / BS) + BS);
 }
 
-template <class T>
-int upload_vec(const std::vector<T> &v, T **d) {
-    *d = nullptr;
-    if (v.empty()) return CPSD_OK;
-    CPSD_TRY(cuda_check(cudaMalloc(d, sizeof(T) * v.size()), "cudaMalloc(short-K plan)"));
-    return cuda_check(cudaMemcpyAsync(*d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, stream()),
-                      "upload short-K plan");
-}
-
 template <int BS, bool FM>
 int launch_one(const ContractPlan *cp, const ShortKPlan *sp, const double *A, const double *B, double *C,
                double alpha) {
@@ -217,7 +208,7 @@ int ShortKPlan::upload() {
     if (uploaded.load(std::memory_order_acquire)) return CPSD_OK;
     std::lock_guard<std::mutex> lock(upload_mutex());
     if (uploaded.load(std::memory_order_relaxed)) return CPSD_OK;
-    CPSD_TRY(upload_vec(items, &d_items));
+    CPSD_TRY(upload_table(items, &d_items, "short-K plan"));
     // the table may next be read by kernels on another thread's stream
     CPSD_TRY(cuda_check(cudaStreamSynchronize(stream()), "plan upload"));
     uploaded.store(true, std::memory_order_release);
