@@ -1671,8 +1671,15 @@ int cpsd_eecpsd_roots(const cpsd_system *s, const cpsd_integrals *I, const cpsd_
         if (per_root * (double)nroot > 0.05 * ctx().mem_share * (double)dev_total) {
             size_t fr = 0, tot_mem = 0;
             CPSD_TRY(cuda_check(cudaMemGetInfo(&fr, &tot_mem), "cudaMemGetInfo"));
+            // three fifths of it: idle pool buffers that the next run asks for
+            // again, the digit tiles of the roots' own operands and the gaps
+            // between scratch chunks need the rest.  D2h nmo 400, 6 digits, ten
+            // roots: three a batch, 592 ms a pipeline without a driver call; at
+            // 0.7 four a batch, which took scratch and tiles from one another by
+            // cudaFree and cudaMalloc in every run (610 ms, up to 642); at 0.4
+            // two, 615 ms.
             const double avail = (double)fr + (double)arena().spare() + (double)pool_idle_bytes();
-            chunk = std::max<i64>(1, std::min<i64>(nroot, (i64)(0.7 * ctx().mem_share * avail / per_root)));
+            chunk = std::max<i64>(1, std::min<i64>(nroot, (i64)(0.6 * ctx().mem_share * avail / per_root)));
         }
     }
     if (getenv("CPSD_TRACE")) {
