@@ -354,6 +354,9 @@ int cpsd_debug_geev(const double *A_host, int64_t n, double *wr, double *wi, dou
  * whose column k is the eigenvector of w[k], of the sign that the order of the
  * rotations gives */
 int cpsd_debug_syev(const double *A_host, int64_t n, double *w, double *V_host);
+/* at most this many CTAs (1..16) in the clusters of the Davidson and DIIS steps
+ * that the calling thread launches, as on a device that holds no larger ones */
+int cpsd_debug_team_cap(int64_t ctas);
 int cpsd_debug_pairmap_plan(const cpsd_opt *in, int64_t op0, int64_t op1, int64_t tgt0, int64_t tgt1,
                             const void **blocks, int64_t *nblocks, const void **idx, const void **sgn,
                             int64_t *nidx, int64_t *lterms, int64_t *rterms);

@@ -1329,6 +1329,12 @@ int cpsd_debug_syev(const double *A_host, int64_t n, double *w, double *V_host) 
     return read_back(V_host, dV, sizeof(double) * n * n);
 }
 
+int cpsd_debug_team_cap(int64_t ctas) {
+    if (ctas < 1 || ctas > 16) return set_error(CPSD_EARG, "cluster sizes are 1..16");
+    ctx().team_cap = (int)ctas;
+    return CPSD_OK;
+}
+
 int64_t cpsd_irpdso(int64_t sym, const int64_t *popp, const int64_t *popq, int64_t ioppq) {
     return irpdso(sym, popp, popq, ioppq);
 }

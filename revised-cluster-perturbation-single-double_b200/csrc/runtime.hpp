@@ -46,6 +46,7 @@ struct Context {
     // fraction of the free device memory this thread may plan its scratch
     // for (molecules running side by side share it)
     double mem_share = 1.0;
+    int team_cap = 16;  // most CTAs of a solver step's cluster (verification)
 };
 Context &ctx();
 inline i64 dp(i64 a, i64 b) { return ctx().dirprd[a - 1][b - 1]; }

@@ -63,38 +63,60 @@ struct Team {
     }
 };
 
-// CTAs of a team: `per` elements each, up to 16 CTAs (of one GPC: above the
-// portable 8)
-int team_size(i64 n, i64 per) {
+// CTAs of a team: `per` elements each, up to `most` CTAs (16, of one GPC: above
+// the portable 8)
+int team_size(i64 n, i64 per, int most) {
     int c = 1;
-    while (c < 16 && (i64)c * per < n) c *= 2;
+    while (2 * c <= most && (i64)c * per < n) c *= 2;
     return c;
 }
 
-template <class... P, class... A>
-int launch_team(void (*kern)(P...), int teams, int size, size_t smem, const char *what, A... args) {
+cudaLaunchConfig_t team_config(int teams, int size, size_t smem, cudaLaunchAttribute *at) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(teams * size));
     cfg.blockDim = dim3(DT);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream();
-    cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)size;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    return cfg;
+}
+template <class... P, class... A>
+int launch_team(void (*kern)(P...), int teams, int size, size_t smem, const char *what, A... args) {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = team_config(teams, size, smem, at);
     return cuda_check(cudaLaunchKernelEx(&cfg, kern, P(args)...), what);
 }
-template <class K>
-int team_attrs(K *kern, size_t smem, std::atomic<bool> &done) {
-    if (done.load(std::memory_order_acquire)) return CPSD_OK;
-    if (smem)
-        CPSD_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                            "solver smem attr"));
-    CPSD_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
-                        "solver cluster attr"));
-    done.store(true, std::memory_order_release);
+// Largest cluster of `kern` with up to smem bytes a CTA that the current device
+// runs: 16 on a whole B200, fewer where part of the SMs is set aside.  Asked
+// once per kernel and device, with the kernel's attributes set.
+constexpr int TEAM_MAXDEV = 64;
+template <class... P>
+int team_most(void (*kern)(P...), size_t smem, std::atomic<int> (&cache)[TEAM_MAXDEV], int *most) {
+    int dev = 0;
+    CPSD_TRY(cuda_check(cudaGetDevice(&dev), "cudaGetDevice"));
+    *most = dev < TEAM_MAXDEV ? cache[dev].load(std::memory_order_acquire) : 0;
+    if (!*most) {
+        if (smem)
+            CPSD_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
+                                "solver smem attr"));
+        CPSD_TRY(cuda_check(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1),
+                            "solver cluster attr"));
+        int size = 16;
+        for (; size > 1; size /= 2) {
+            cudaLaunchAttribute at[1];
+            const cudaLaunchConfig_t cfg = team_config(1, size, smem, at);
+            int active = 0;
+            if (cudaOccupancyMaxActiveClusters(&active, kern, &cfg) == cudaSuccess && active > 0) break;
+            cudaGetLastError();  // a size that the device refuses
+        }
+        *most = size;
+        if (dev < TEAM_MAXDEV) cache[dev].store(size, std::memory_order_release);
+    }
+    *most = std::min(*most, ctx().team_cap);
     return CPSD_OK;
 }
 
@@ -1761,11 +1783,12 @@ int dav_init_launch(DavState *st, const DavBuffers &b) {
 int dav_step_launch(DavState *st, const DavBuffers &b, i64 n, int nroot, int D) {
     constexpr size_t base = (sizeof(DavShared) + 15) / 16 * 16, most = base + sizeof(double) * DAV_LOCAL;
     static_assert(most + 1024 <= 227 * 1024, "shared memory of a Davidson step");
-    static std::atomic<bool> attr{false};
-    CPSD_TRY(team_attrs(k_dav_step, most, attr));
+    static std::atomic<int> fits[TEAM_MAXDEV];
+    int ctas;
+    CPSD_TRY(team_most(k_dav_step, most, fits, &ctas));
     cudaEvent_t end;
     CPSD_TRY(timing_begin(0.0, 0, 0, 0, 30, &end));
-    const int size = team_size(n, DAV_PER);
+    const int size = team_size(n, DAV_PER, ctas);
     const int nc = (int)(((n + size - 1) / size + 31) & ~(i64)31);
     const i64 need = (i64)2 * (D + nroot) * dav_ld(nc);
     const int local = need <= DAV_LOCAL;
@@ -1791,11 +1814,12 @@ int dav_final_launch(DavState *st, const DavBuffers &b) {
 }
 int solver_step_launch(const SolverArgs &a) {
     if (a.nb <= 0) return CPSD_OK;
-    static std::atomic<bool> attr{false};
-    CPSD_TRY(team_attrs(k_solver_step, 0, attr));
+    static std::atomic<int> fits[TEAM_MAXDEV];
+    int ctas;
+    CPSD_TRY(team_most(k_solver_step, 0, fits, &ctas));
     cudaEvent_t end;
     CPSD_TRY(timing_begin(0.0, a.nb, 0, 0, 32, &end));
-    CPSD_TRY(launch_team(k_solver_step, a.nb, team_size(a.len, DT), 0, "k_solver_step", a));
+    CPSD_TRY(launch_team(k_solver_step, a.nb, team_size(a.len, DT, ctas), 0, "k_solver_step", a));
     count_launch();
     return timing_end(end);
 }

@@ -70,3 +70,26 @@ def test_diis_loop_matches_oracle(nmo, nocc_a, nirrep):
     assert g["iters"] == r["iters"]
     assert np.linalg.norm(t - ref) < 1e-9 * np.linalg.norm(ref)
     assert abs(g["E3"] - r["E3"]) < 1e-11 * max(1.0, abs(r["E3"]))
+
+
+@pytest.mark.parametrize("cap", [1, 2, 4, 8])
+def test_smaller_clusters(cap):
+    """A device that holds only smaller clusters: the same roots and amplitudes from fewer CTAs."""
+    s = synth.System(nmo=60, nocc_a=9, nocc_b=7, nirrep=1, seed=5, roots=3,
+                     run_opts=dict(lowest=1, davidson_conv=9, davidson_cyc=100))
+    for x in s.ints.values():  # the singles equations converge, as above
+        x *= 0.1
+    api.use_torch_stream()
+    ints, sysc, par = api.DeviceIntegrals(s), api.make_system(s), api.make_params(s)
+    om, R, _ = api.cis_run(s, sysc, ints, par)
+    g = api.ground(s, sysc, ints, par)
+    api.check(api.lib().cpsd_debug_team_cap(api.I64(cap)), "cap")
+    try:
+        om1, R1, _ = api.cis_run(s, sysc, ints, par)
+        g1 = api.ground(s, sysc, ints, par)
+    finally:
+        api.check(api.lib().cpsd_debug_team_cap(api.I64(16)), "cap")
+    assert np.max(np.abs(om1 - om)) < 1e-11
+    assert float((R1 - R).abs().max()) < 1e-7
+    assert g["iters"] == g1["iters"]
+    assert float((g1["T1_2"] - g["T1_2"]).norm()) < 1e-9 * float(g["T1_2"].norm())
