@@ -375,7 +375,10 @@ int o_davidson(double *fileEV, const double *diagA, i64 dimA, i64 nroot, i64 ist
                const o_params *p, o_sigma_fn calAR, void *ctx, i64 *iters_out)
 {
     i64 dimAbar = p->davidson_dim;
+    /* a collapse keeps nroot + 5 vectors, the roots alone where that would be
+     * the whole basis or more */
     i64 dimDel = dimAbar - nroot - 5;
+    if (dimDel < 1) dimDel = dimAbar - nroot;
     if (nroot >= dimAbar) return O_EARG;
     if (nroot == 0) return O_OK;
     double maxError = pow(10.0, -(double)p->davidson_conv);

@@ -295,7 +295,10 @@ int davidson(const cpsd_params *p, i64 n, i64 nroot, double *fileEV, const doubl
     hs.nroot = (int)nroot;
     hs.lowest = (int)p->lowest;
     hs.maxcyc = (int)p->davidson_cyc;
-    hs.dimDel = (int)(D - nroot - 5);
+    // vectors that a collapse of the full basis leaves out: the reference keeps
+    // nroot + 5 (mod_davidson.f90:266-325); where that is the whole basis or more,
+    // the roots alone are kept
+    hs.dimDel = (int)(D - nroot - 5 > 0 ? D - nroot - 5 : D - nroot);
     hs.maxError = std::pow(10.0, -(double)p->davidson_conv);
     DavState *st;
     CPSD_TRY(arena().alloc(sizeof(DavState), (void **)&st));

@@ -38,7 +38,11 @@ def test_cis_roots_match_dense(nmo, nocc_a, nirrep, roots):
     api.use_torch_stream()
     ints = api.DeviceIntegrals(s)
     om, R, it = api.cis_run(s, api.make_system(s), ints, api.make_params(s))
-    # the spin-flip block: alpha occupied to beta virtual
+    check_cis(s, om, R, roots)
+
+
+def check_cis(s, om, R, roots):
+    """roots against dense diagonalisation of the spin-flip block: alpha occupied to beta virtual"""
     o, v = int(s.popo.sum()), int(s.popv.sum())
     n = o * v
     V = torch.from_numpy(s.ints["iabj"]).cuda().view(n, n)  # element (fn, ai) of the column-major block: row (ai)
@@ -53,6 +57,19 @@ def test_cis_roots_match_dense(nmo, nocc_a, nirrep, roots):
     assert float(res.abs().max()) < 1e-9
     G = X @ X.T
     assert float((G - torch.eye(roots, dtype=torch.float64, device="cuda")).abs().max()) < 1e-8
+
+
+# basis, roots: a collapse that keeps roots + 5, then those where that is the whole basis or more (the roots are kept)
+@pytest.mark.parametrize("dim,roots", [(20, 14), (20, 15), (20, 16), (20, 19), (32, 27), (32, 28), (32, 31)])
+@pytest.mark.parametrize("nmo", [28, 101])  # 384 elements: four CTAs, in shared memory; 3960: 16, in global memory
+def test_many_roots_in_a_small_basis(nmo, dim, roots):
+    s = synth.System(nmo=nmo, nocc_a=5 if nmo < 50 else 12, nocc_b=3 if nmo < 50 else 10, nirrep=1, seed=3, roots=roots,
+                     skip_abcd=True,
+                     run_opts=dict(lowest=1, davidson_conv=10, davidson_cyc=3000, davidson_dim=dim))
+    s.ints["iabj"] *= 0.02 if nmo < 50 else 0.004  # one to six free places: weakly coupled configurations converge
+    api.use_torch_stream()
+    om, R, _ = api.cis_run(s, api.make_system(s), api.DeviceIntegrals(s), api.make_params(s))
+    check_cis(s, om, R, roots)
 
 
 @pytest.mark.parametrize("nmo,nocc_a,nirrep", [(28, 5, 1), (44, 8, 1), (44, 9, 1), (80, 14, 2)])
