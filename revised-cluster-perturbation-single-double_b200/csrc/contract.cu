@@ -520,7 +520,8 @@ int launch_tiles(const ContractPlan *p, const double *A, const double *B, double
         // a caller's workspace may hold no more than the fixed rule asks for
         // (K parts of 256 and more): the same contraction with those tiles
         const ContractPlan *q = nullptr;
-        if (rc != CPSD_OK && arena().external && plan_fixed(p, &q) == CPSD_OK && q->nparts < p->nparts)
+        if (rc != CPSD_OK && arena().external && plan_fixed(p, &q) == CPSD_OK &&
+            q->nparts * TILE_BM[q->shape()] * TILE_BN[q->shape()] < p->nparts * bm * bn)
             return launch_tiles(q, A, B, C, alpha);
         CPSD_TRY(rc);
     }
