@@ -866,14 +866,12 @@ int vjp444(const Ten &v1, const Ten &v2, const Ten &Y, Ten &G, int which, double
 }
 
 namespace {
-// A packed (vv|vo) list times singles by the kernels that read it packed,
-// unless the mixed mode would send the expanded contraction to the digit
-// path (*done stays false: the caller takes the general path).  No expanded
-// copy is made or kept.
+// A packed (vv|vo) list times singles by the kernels that read it packed
+// (`takes` checked by the caller), unless the mixed mode would send the
+// expanded contraction to the digit path (*done stays false: the caller takes
+// the general path).  No expanded copy is made or kept.
 int packed_singles(const Ten &V, const char *tv, const Ten &r, const char *tr, Ten &out, const char *to, i64 nb,
                    int (*run)(const Ten &, const Ten &, Ten &, double, i64, bool *), double f, bool *done) {
-    CPSD_TRY(need_init());
-    if (V.d.iop[0] != 0) return CPSD_OK;
     OpScope op;
     Desc full = V.d;
     full.iop[0] = 1;
@@ -1038,7 +1036,9 @@ int k_Fmi_r1ijka(Ten &F, const Ten &r1, const Ten &V, double f, i64 nb) {
 }
 int k_Fae_r1abci(Ten &F, const Ten &r1, const Ten &V, double f, i64 nb) {
     bool done = false;
-    CPSD_TRY(packed_singles(V, "efam", r1, "fm+-", F, "ae+-", nb, pairblk_fae, f, &done));
+    CPSD_TRY(need_init());
+    if (pairblk_fae_takes(V, r1, F, nb))
+        CPSD_TRY(packed_singles(V, "efam", r1, "fm+-", F, "ae+-", nb, pairblk_fae, f, &done));
     if (done) return CPSD_OK;
     return w422(V, r1, F, f, "efam", "fm", "ae", nb);
 }
@@ -1068,7 +1068,9 @@ int k_Wmbej_r2abij(Ten &W, const Ten &r2, const Ten &V, double f, i64 nb) {
 }
 int k_Wmbej_r1abci(Ten &W, const Ten &r1, const Ten &V, double f, i64 nb) {
     bool done = false;
-    CPSD_TRY(packed_singles(V, "febm", r1, "fj..", W, "embj", nb, pairblk_wmbej, f, &done));
+    CPSD_TRY(need_init());
+    if (pairblk_wmbej_takes(V, r1, W, nb))
+        CPSD_TRY(packed_singles(V, "febm", r1, "fj..", W, "embj", nb, pairblk_wmbej, f, &done));
     if (done) return CPSD_OK;
     return w424(V, r1, W, f, "febm", "fj", "embj", 0, nb);
 }

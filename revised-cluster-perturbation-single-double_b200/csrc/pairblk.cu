@@ -334,14 +334,22 @@ int PairBlkPlan::upload() {
     return CPSD_OK;
 }
 
+bool pairblk_wmbej_takes(const Ten &V, const Ten &r, const Ten &W, i64 nb) {
+    const Desc &v = V.d, &s = r.d, &w = W.d;
+    return layouts_ok(V, r) && w.sym == s.sym && w.iop[0] == 1 && w.iop[1] == 1 && same_pop(w.pop[0], v.pop[0]) &&
+           same_pop(w.pop[1], v.pop[3]) && same_pop(w.pop[2], v.pop[2]) && same_pop(w.pop[3], s.pop[1]) &&
+           !(nb > 1 && r.bs == 0);
+}
+
+bool pairblk_fae_takes(const Ten &V, const Ten &r, const Ten &F, i64 nb) {
+    const Desc &v = V.d, &s = r.d, &w = F.d;
+    return layouts_ok(V, r) && w.sym == s.sym && w.iop[0] == 1 && w.iop[1] == 1 && same_pop(w.pop[0], v.pop[0]) &&
+           same_pop(w.pop[1], v.pop[0]) && is_zorb8(w.pop[2]) && is_zorb8(w.pop[3]) && !(nb > 1 && r.bs == 0);
+}
+
 int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, bool *done) {
     *done = false;
     const Desc &v = V.d, &s = r.d, &w = W.d;
-    if (!layouts_ok(V, r) || w.sym != s.sym || w.iop[0] != 1 || w.iop[1] != 1) return CPSD_OK;
-    if (!same_pop(w.pop[0], v.pop[0]) || !same_pop(w.pop[1], v.pop[3]) || !same_pop(w.pop[2], v.pop[2]) ||
-        !same_pop(w.pop[3], s.pop[1]))
-        return CPSD_OK;
-    if (nb > 1 && r.bs == 0) return CPSD_OK;
     static std::map<std::string, std::unique_ptr<PairBlkPlan>> cache;
     static std::mutex mx;
     PairBlkPlan *p;
@@ -414,10 +422,6 @@ int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, bool *do
 int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, bool *done) {
     *done = false;
     const Desc &v = V.d, &s = r.d, &w = F.d;
-    if (!layouts_ok(V, r) || w.sym != s.sym || w.iop[0] != 1 || w.iop[1] != 1) return CPSD_OK;
-    if (!same_pop(w.pop[0], v.pop[0]) || !same_pop(w.pop[1], v.pop[0]) || !is_zorb8(w.pop[2]) || !is_zorb8(w.pop[3]))
-        return CPSD_OK;
-    if (nb > 1 && r.bs == 0) return CPSD_OK;
     static std::map<std::string, std::unique_ptr<PairBlkPlan>> cache;
     static std::mutex mx;
     PairBlkPlan *p;

@@ -44,9 +44,12 @@ struct PairBlkPlan {
     int upload();
 };
 
+// whether the layouts are those of a packed (vv|vo) list, a singles vector and a
+// full (vo|vo) result, or (vv) result; the calls below take no others
+bool pairblk_wmbej_takes(const Ten &V, const Ten &r, const Ten &W, i64 nb);
+bool pairblk_fae_takes(const Ten &V, const Ten &r, const Ten &F, i64 nb);
 // W(em,bj) += f r(f,j) V(fe,bm) for nb roots; *done = false (and nothing
-// queued) when the layouts are not those of a packed (vv|vo) list, a singles
-// vector and a full (vo|vo) result
+// queued) when the sizes are beyond the kernel's
 int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, bool *done);
 // F(a,e) += f r(f,m) V(ef,am)
 int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, bool *done);

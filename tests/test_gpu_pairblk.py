@@ -56,3 +56,29 @@ def test_packed_pair_matches_oracle(name, nmo, nocc, nirrep, symr):
         api.contract_timing(False)
     assert 23 in kinds and 40 not in kinds, "the list was expanded"
     assert float(np.max(np.abs(dev[0].cpu().numpy() - ref))) < 2e-12 * (1 + np.max(np.abs(ref)) / 50)
+
+
+@pytest.mark.parametrize("name", ["Wmbej_r1abci", "Fae_r1abci"])
+def test_second_pair_packed(name):
+    """A list whose second pair is packed too (its two spaces of the same populations) is a call of the general path,
+    which expands both pairs: the result is that of the list with the second pair full."""
+    n, rng = 6, np.random.default_rng(1)
+    p, z = np.array([n] + [0] * 7, np.int64), np.array([1] + [0] * 7, np.int64)
+    api.use_torch_stream()
+    api.init(1, np.ones((8, 8), np.int64))
+    np2 = n * (n - 1) // 2
+    packed = rng.standard_normal((np2, np2))  # column (x, m), x < m; rows (p, q), p < q
+    full = np.zeros((n, n, np2))
+    cols = [(x, m) for m in range(n) for x in range(m)]
+    for k, (x, m) in enumerate(cols):
+        full[m, x], full[x, m] = packed[k], -packed[k]
+    r = torch.from_numpy(rng.standard_normal(n * n)).cuda()
+    pops = [p, p, p, p] if name[0] == "W" else [p, p, z, z]
+    got = []
+    for iop, x in ((0, packed), (1, full)):
+        out = torch.zeros(int(np.prod([q.sum() for q in pops])), dtype=torch.float64, device="cuda")
+        api.kernel(name, api.opt(pops, (1, 1), 1, out), api.opt([p, p, z, z], (1, 1), 1, r),
+                   api.opt([p] * 4, (0, iop), 1, torch.from_numpy(x.reshape(-1).copy()).cuda()), 0.7)
+        got.append(out)
+    assert float(got[1].abs().max()) > 0.1
+    assert float((got[0] - got[1]).abs().max()) < 1e-13  # sums of up to 36 products of size 1
