@@ -871,7 +871,7 @@ namespace {
 // expanded contraction to the digit path (*done stays false: the caller takes
 // the general path).  No expanded copy is made or kept.
 int packed_singles(const Ten &V, const char *tv, const Ten &r, const char *tr, Ten &out, const char *to, i64 nb,
-                   int (*run)(const Ten &, const Ten &, Ten &, double, i64, bool *), double f, bool *done) {
+                   int (*run)(const Ten &, const Ten &, Ten &, double, i64, double, bool *), double f, bool *done) {
     OpScope op;
     Desc full = V.d;
     full.iop[0] = 1;
@@ -887,7 +887,7 @@ int packed_singles(const Ten &V, const char *tv, const Ten &r, const char *tr, T
     const OzPlan *oz = nullptr;
     CPSD_TRY(digit_route(p, &oz));
     if (oz) return CPSD_OK;
-    CPSD_TRY(run(V, r, out, f, nb, done));
+    CPSD_TRY(run(V, r, out, f, nb, p->flops, done));
     if (*done) {
         trace_contraction(p, tv, tr, to, nb, "packed pair");
         ctx().flops += p->flops;

@@ -347,7 +347,7 @@ bool pairblk_fae_takes(const Ten &V, const Ten &r, const Ten &F, i64 nb) {
            same_pop(w.pop[1], v.pop[0]) && is_zorb8(w.pop[2]) && is_zorb8(w.pop[3]) && !(nb > 1 && r.bs == 0);
 }
 
-int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, bool *done) {
+int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, double flops, bool *done) {
     *done = false;
     const Desc &v = V.d, &s = r.d, &w = W.d;
     static std::map<std::string, std::unique_ptr<PairBlkPlan>> cache;
@@ -411,7 +411,7 @@ int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, bool *do
     if (p->groups.empty()) return CPSD_OK;
     CPSD_TRY(p->upload());
     cudaEvent_t end;
-    CPSD_TRY(timing_begin(0.0, (i64)p->groups.size(), p->items * ncg, W.len() * nb, 23, &end));
+    CPSD_TRY(timing_begin(flops, (i64)p->groups.size(), p->items * ncg, W.len() * nb, 23, &end));
     const i64 wb = nb > 1 ? (W.bs ? W.bs : W.len()) : 0;
     if (p->maxp <= 32) CPSD_TRY(wmbej_go<4>(*p, V, r, W, f, nb, wb));
     else if (p->maxp <= 64) CPSD_TRY(wmbej_go<8>(*p, V, r, W, f, nb, wb));
@@ -419,7 +419,7 @@ int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, bool *do
     return timing_end(end);
 }
 
-int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, bool *done) {
+int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, double flops, bool *done) {
     *done = false;
     const Desc &v = V.d, &s = r.d, &w = F.d;
     static std::map<std::string, std::unique_ptr<PairBlkPlan>> cache;
@@ -470,7 +470,7 @@ int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, bool *done
     if (p->groups.empty()) return CPSD_OK;
     CPSD_TRY(p->upload());
     cudaEvent_t end;
-    CPSD_TRY(timing_begin(0.0, (i64)p->groups.size(), p->nrow, F.len() * nb, 23, &end));
+    CPSD_TRY(timing_begin(flops, (i64)p->groups.size(), p->nrow, F.len() * nb, 23, &end));
     const i64 fb = nb > 1 ? (F.bs ? F.bs : F.len()) : 0;
     if (p->maxp <= 32) CPSD_TRY(fae_go<4>(*p, V, r, F, f, nb, fb));
     else if (p->maxp <= 64) CPSD_TRY(fae_go<8>(*p, V, r, F, f, nb, fb));

@@ -49,9 +49,10 @@ struct PairBlkPlan {
 bool pairblk_wmbej_takes(const Ten &V, const Ten &r, const Ten &W, i64 nb);
 bool pairblk_fae_takes(const Ten &V, const Ten &r, const Ten &F, i64 nb);
 // W(em,bj) += f r(f,j) V(fe,bm) for nb roots; *done = false (and nothing
-// queued) when the sizes are beyond the kernel's
-int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, bool *done);
+// queued) when the sizes are beyond the kernel's.  flops: of the contraction,
+// for the timing record
+int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, double flops, bool *done);
 // F(a,e) += f r(f,m) V(ef,am)
-int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, bool *done);
+int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, double flops, bool *done);
 
 }  // namespace cpsd

@@ -82,3 +82,22 @@ def test_second_pair_packed(name):
         got.append(out)
     assert float(got[1].abs().max()) > 0.1
     assert float((got[0] - got[1]).abs().max()) < 1e-13  # sums of up to 36 products of size 1
+
+
+@pytest.mark.parametrize("name", ["Wmbej_r1abci", "Fae_r1abci"])
+def test_records_hold_the_flops(name):
+    n, z = 20, np.array([1] + [0] * 7, np.int64)
+    v, o = np.array([n] + [0] * 7, np.int64), np.array([3] + [0] * 7, np.int64)
+    api.use_torch_stream()
+    api.init(1, np.ones((8, 8), np.int64))
+    pops = [v, o, v, o] if name[0] == "W" else [v, v, z, z]
+    t = [torch.ones(m, dtype=torch.float64, device="cuda")
+         for m in (int(np.prod([q.sum() for q in pops])), 3 * n, n * (n - 1) // 2 * 3 * n)]
+    ops = [api.opt(pops, (1, 1), 1, t[0]), api.opt([v, o, z, z], (1, 1), 1, t[1]), api.opt([v, v, v, o], (0, 1), 1, t[2])]
+    api.contract_timing(True)
+    try:
+        api.kernel(name, *ops, 0.7)
+        _, flops, kinds, _ = api.contract_records()
+    finally:
+        api.contract_timing(False)
+    assert 2.0 * n * 3 * n * n * (3 if name[0] == "W" else 1) in [f for f, k in zip(flops, kinds) if k == 23]
