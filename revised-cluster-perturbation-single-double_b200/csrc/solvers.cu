@@ -816,7 +816,7 @@ struct DavShared {
 };
 
 // The basis, its sigma vectors and the work vectors of a step live in shared
-// memory when this many doubles hold a CTA's part of them (n up to about 3900
+// memory when this many doubles hold a CTA's part of them (n up to 4096
 // with 16 CTAs, a basis of 20 and 5 roots): copied there while the Ritz
 // problem is solved, they cost one latency instead of one for each of the
 // step's eight passes.

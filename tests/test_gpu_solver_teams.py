@@ -30,7 +30,8 @@ pytestmark = pytest.mark.gpu
     (48, 9, 1, 5),    # 1280: eight CTAs
     (85, 10, 1, 4),   # 2736: 16 CTAs, vectors in shared memory
     (85, 10, 1, 12),  # the same, vectors in global memory
-    (101, 12, 1, 2),  # 3960: 16 CTAs, longer than the shared memory holds
+    (101, 12, 1, 2),  # 3960: 16 CTAs, in shared memory
+    (105, 12, 1, 5),  # 4136: longer than the shared memory holds, collapses of ten vectors
 ])
 def test_cis_roots_match_dense(nmo, nocc_a, nirrep, roots):
     s = synth.System(nmo=nmo, nocc_a=nocc_a, nocc_b=nocc_a - 2, nirrep=nirrep, seed=3, roots=roots, skip_abcd=True,
@@ -72,9 +73,10 @@ def test_many_roots_in_a_small_basis(nmo, dim, roots):
     check_cis(s, om, R, roots)
 
 
-@pytest.mark.parametrize("nmo,nocc_a,nirrep", [(28, 5, 1), (44, 8, 1), (44, 9, 1), (80, 14, 2)])
+@pytest.mark.parametrize("nmo,nocc_a,nirrep", [(28, 5, 1), (36, 6, 1), (44, 8, 1), (44, 9, 1), (80, 14, 2), (56, 16, 1),
+                                               (72, 24, 1)])
 def test_diis_loop_matches_oracle(nmo, nocc_a, nirrep):
-    """T1^(2) vectors of 384, 1036 (two CTAs), 1152 and 1744 elements"""
+    """T1^(2) vectors of 384 elements (one CTA), 620 (two), 1036, 1152 and 1744 (four), 2460 (eight), 4508 (16)"""
     s = synth.System(nmo=nmo, nocc_a=nocc_a, nocc_b=nocc_a - 2, nirrep=nirrep, seed=4, roots=1)
     # weaker integrals keep the singles equations definite at these sizes, so that the loop converges
     for k, x in s.ints.items():
