@@ -99,7 +99,7 @@ int plan_eri_list(const Sys &S, int which, const EriListPlan **out) {
     static std::mutex m;
     std::lock_guard<std::mutex> lock(m);
     static std::map<std::string, std::unique_ptr<EriListPlan>> cache;
-    std::string key = std::to_string(which) + "#" + std::to_string(ctx().nirrep);
+    std::string key = std::to_string(which) + sym_key();
     for (int h = 0; h < 8; h++) key += "," + std::to_string(S.popo[h]) + "," + std::to_string(S.popv[h]);
     auto it = cache.find(key);
     if (it != cache.end()) {

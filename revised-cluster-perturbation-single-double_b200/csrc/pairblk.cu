@@ -353,7 +353,7 @@ int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, double f
     static std::map<std::string, std::unique_ptr<PairBlkPlan>> cache;
     static std::mutex mx;
     PairBlkPlan *p;
-    CPSD_TRY(cached(cache, mx, v.key() + s.key() + w.key() + std::to_string(ctx().nirrep), &p, [&](PairBlkPlan &P) {
+    CPSD_TRY(cached(cache, mx, v.key() + s.key() + w.key() + sym_key(), &p, [&](PairBlkPlan &P) {
         const i64 n = ctx().nirrep;
         const i64 *pv = v.pop[0], *po = v.pop[3];
         for (i64 hx = 1; hx <= n; hx++)
@@ -425,7 +425,7 @@ int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, double flo
     static std::map<std::string, std::unique_ptr<PairBlkPlan>> cache;
     static std::mutex mx;
     PairBlkPlan *p;
-    CPSD_TRY(cached(cache, mx, v.key() + s.key() + w.key() + std::to_string(ctx().nirrep), &p, [&](PairBlkPlan &P) {
+    CPSD_TRY(cached(cache, mx, v.key() + s.key() + w.key() + sym_key(), &p, [&](PairBlkPlan &P) {
         const i64 n = ctx().nirrep;
         const i64 *pv = v.pop[0], *po = v.pop[3];
         for (i64 ha = 1; ha <= n; ha++) {

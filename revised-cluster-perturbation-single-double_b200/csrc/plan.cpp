@@ -239,7 +239,7 @@ int plan_contract(const Desc &d1, const char *t1, const Desc &d2, const char *t2
     static std::map<std::string, std::unique_ptr<ContractPlan>> cache;
     std::string key = d1.key() + t1 + d2.key() + t2 + d3.key() + t3 + "#" + std::to_string(batch.nb) + "," +
                       std::to_string(batch.strideA) + "," + std::to_string(batch.strideB) + "," +
-                      std::to_string(batch.strideC) + "#" + std::to_string(ctx().nirrep);
+                      std::to_string(batch.strideC) + sym_key();
     auto it = cache.find(key);
     if (it != cache.end()) {
         *out = it->second.get();
@@ -663,7 +663,7 @@ int plan_pairmap(const Desc &din, int op0, int op1, i64 target_iop0, i64 target_
     }
     *dout_ret = dout;
     std::string key = din.key() + "|" + std::to_string(op0) + std::to_string(op1) + std::to_string(target_iop0) +
-                      std::to_string(target_iop1) + "#" + std::to_string(ctx().nirrep);
+                      std::to_string(target_iop1) + sym_key();
     auto it = cache.find(key);
     if (it != cache.end()) {
         *out = it->second.get();
@@ -744,7 +744,7 @@ int plan_energy(const Desc &d, const char *kinds, const EnergyPlan **out) {
     static std::mutex m;
     std::lock_guard<std::mutex> lock(m);
     static std::map<std::string, std::unique_ptr<EnergyPlan>> cache;
-    std::string key = d.key() + kinds + "#" + std::to_string(ctx().nirrep);
+    std::string key = d.key() + kinds + sym_key();
     auto it = cache.find(key);
     if (it != cache.end()) {
         *out = it->second.get();

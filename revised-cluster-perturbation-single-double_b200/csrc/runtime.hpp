@@ -50,6 +50,9 @@ struct Context {
 };
 Context &ctx();
 inline i64 dp(i64 a, i64 b) { return ctx().dirprd[a - 1][b - 1]; }
+// the symmetry as part of a plan's key: irreps and their products (tables of
+// eight irreps differ with the order of the irreps)
+std::string sym_key();
 inline cudaStream_t stream() { return ctx().stream; }
 inline void count_launch(int n = 1) { ctx().launches += n; }
 

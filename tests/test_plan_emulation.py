@@ -13,9 +13,11 @@ import ctypes
 import numpy as np
 import pytest
 
+import dense
 import kernel_specs as ks
 import oracle_ffi as of
 from cpsd_b200 import api, synth
+from cpsd_b200.dpd import Symmetry, xor_dirprd
 
 I64 = ctypes.c_int64
 MAXU = 4
@@ -319,3 +321,29 @@ def test_pairmap_plans_in_bounds_and_match_oracle(nirrep):
             y2 = y1 - sw2
             lib.o_icompso(of.ptr(y2), of.ptr(ref), ctypes.byref(din), I64(0), I64(0))
         np.testing.assert_allclose(out, ref, rtol=0, atol=1e-13)
+
+
+def test_plans_follow_the_product_table():
+    """Eight irreps in another order have another product table: plans of one are not those of the other."""
+    xor = np.array(xor_dirprd(8)).reshape(8, 8)
+    perm = np.array([0, 1, 2, 4, 3, 5, 6, 7])  # the product of 2 and 3 is 4 in one order and 5 in the other
+    inv = np.argsort(perm)
+    other = np.ascontiguousarray([[perm[xor[inv[i], inv[j]] - 1] + 1 for j in range(8)] for i in range(8)], np.int64)
+    rng = np.random.default_rng(0)
+    pops = [np.array(p, np.int64) for p in ([3, 1, 2, 1, 2, 3, 1, 2], [1, 2, 1, 2, 1, 1, 2, 1])]
+    v, o = pops
+    spec = (("aebf", [v, v, v, v]), ("eifj", [v, o, v, o]), ("aibj", [v, o, v, o]))
+    for table in (xor, other):
+        api.init(8, table)
+        sym = Symmetry(8, table)
+        opts, x = [], []
+        for _, p in spec:
+            opt = api.Opt()
+            api.check(api.lib().cpsd_opt_init(ctypes.byref(opt), *[api.arr8(q) for q in p], I64(1), I64(1), I64(1), None),
+                      "opt")
+            opts.append(opt)
+            x.append(rng.standard_normal(sym.idsymsoc(1, p[0], p[1], 1, p[2], p[3], 1)))
+        tasks, segs, tiles, tile = get_plan(opts[0], spec[0][0], opts[1], spec[1][0], opts[2], spec[2][0])
+        got = emulate(tasks, segs, tiles, x[0], x[1], x[2], 1.0, tile)
+        d = [dense.dpd_to_dense(y, sym, p, (1, 1), 1) for y, (_, p) in zip(x + [got], spec + spec[2:])]
+        np.testing.assert_allclose(d[3], d[2] + np.einsum("aebf,eifj->aibj", d[0], d[1]), rtol=0, atol=1e-12)
