@@ -413,9 +413,11 @@ int pairblk_wmbej(const Ten &V, const Ten &r, Ten &W, double f, i64 nb, double f
     cudaEvent_t end;
     CPSD_TRY(timing_begin(flops, (i64)p->groups.size(), p->items * ncg, W.len() * nb, 23, &end));
     const i64 wb = nb > 1 ? (W.bs ? W.bs : W.len()) : 0;
-    if (p->maxp <= 32) CPSD_TRY(wmbej_go<4>(*p, V, r, W, f, nb, wb));
-    else if (p->maxp <= 64) CPSD_TRY(wmbej_go<8>(*p, V, r, W, f, nb, wb));
-    else CPSD_TRY(wmbej_go<12>(*p, V, r, W, f, nb, wb));
+    // strips of 32 rows at every size: with 4, 8 and 12 row tiles of 8 the
+    // launch took 22, 33, 39 us at 32 rows an irrep (C2v, 12 occupied), 55, 59,
+    // 70 at 48, 88, 94, 115 at 64, 148, 172, 154 at 72, 254, 307, 258 at 96,
+    // 336, 342, 404 at 97, 555, 549, 675 at 128; 72, 68, 74 at 160 without symmetry
+    CPSD_TRY(wmbej_go<4>(*p, V, r, W, f, nb, wb));
     return timing_end(end);
 }
 
@@ -465,16 +467,19 @@ int pairblk_fae(const Ten &V, const Ten &r, Ten &F, double f, i64 nb, double flo
         }
         P.glist.push_back((int)P.groups.size());
     }));
-    if (pb_smem<12>() + sizeof(double) * PW * 8 * (size_t)p->maxe > PB_SMEM_MOST) return CPSD_OK;
+    if (pb_smem<8>() + sizeof(double) * PW * 8 * (size_t)p->maxe > PB_SMEM_MOST) return CPSD_OK;
     *done = true;
     if (p->groups.empty()) return CPSD_OK;
     CPSD_TRY(p->upload());
     cudaEvent_t end;
     CPSD_TRY(timing_begin(flops, (i64)p->groups.size(), p->nrow, F.len() * nb, 23, &end));
     const i64 fb = nb > 1 ? (F.bs ? F.bs : F.len()) : 0;
+    // 4, 8 and 12 row tiles, us a launch: 18, 21, 27 at 32 rows an irrep (C2v),
+    // 38, 35, 47 at 48, 51, 45, 59 at 64, 74, 74, 71 at 72, 115, 117, 119 at 96,
+    // 150, 129, 180 at 97, 285, 279, 336 at 128; 94, 104, 109 at 160 without
+    // symmetry.  Two instances come within a tenth of the best everywhere.
     if (p->maxp <= 32) CPSD_TRY(fae_go<4>(*p, V, r, F, f, nb, fb));
-    else if (p->maxp <= 64) CPSD_TRY(fae_go<8>(*p, V, r, F, f, nb, fb));
-    else CPSD_TRY(fae_go<12>(*p, V, r, F, f, nb, fb));
+    else CPSD_TRY(fae_go<8>(*p, V, r, F, f, nb, fb));
     return timing_end(end);
 }
 

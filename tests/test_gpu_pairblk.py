@@ -1,8 +1,8 @@
 """The kernels that read the packed (vv|vo) list (Wmbej_r1abci, Fae_r1abci)
-against the oracle where they can go wrong: one to three chunks of 96 rows
-with remainders, row tiles of 8 and strips of 8 at and beside their edges,
+against the oracle where they can go wrong: one to seven chunks of 32 (64)
+rows with remainders, row tiles of 8 and strips of 8 at and beside their edges,
 more than eight columns, singles of another irrep than 1, irreps without
-occupied orbitals, every tile-count instance.
+occupied orbitals, both tile-count instances.
 
 Operands are standard normal, so an output is a sum of at most 2 x 212 terms of
 size 1: its FP64 rounding is below 424 eps sqrt(424) = 2e-12, in either order.
@@ -20,11 +20,11 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("name", ["Wmbej_r1abci", "Fae_r1abci"])
 @pytest.mark.parametrize("nmo,nocc,nirrep,symr", [
-    (110, (3, 1), 1, 1),   # v = 216: three chunks
-    (52, (5, 3), 1, 1),    # v = 96: one full chunk
+    (110, (3, 1), 1, 1),   # v = 216: seven chunks of 32, four of 64
+    (52, (5, 3), 1, 1),    # v = 96: three full chunks of 32
     (53, (5, 4), 1, 1),    # v = 97, nine columns
-    (20, (4, 2), 1, 1),    # v = 34: the 8-tile instance
-    (13, (2, 1), 1, 1),    # v = 23: the 4-tile instance
+    (20, (4, 2), 1, 1),    # v = 34: two rows past a chunk of 32
+    (13, (2, 1), 1, 1),    # v = 23: less than a chunk
     (90, (7, 5), 2, 2),    # irreps of 84, singles of irrep 2
     (37, (5, 3), 4, 3),
     (35, (3, 1), 8, 1),    # irreps without occupied orbitals
