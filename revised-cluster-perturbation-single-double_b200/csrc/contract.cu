@@ -8,8 +8,8 @@
 // tensor pipe with mma.sync.m8n8k4.f64 (tcgen05 has no FP64 kind).  K stages
 // of 16 are copied with cp.async into a ring, two or three stages ahead of
 // the one that is multiplied, one barrier a stage; staging them in registers
-// one stage ahead was slower in every shape (128x32 on the C1 nmo-71 ladder:
-// 517 us against 256).  Split-K tiles write
+// one stage ahead was slower in every shape (twice the time with 128x32 on the
+// C1 nmo-71 ladder).  Split-K tiles write
 // partial sums that k_splitk_reduce adds in a fixed order, so results are
 // deterministic.
 #include <atomic>
@@ -147,6 +147,10 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
         // one contracted unit: offsets in a constant step, no table
         const bool afast = sg.aMfast, bfast = sg.bKfast, lin = sg.nk == 1;
         const i64 ksa = sg.kSA[0], ksb = sg.kSB[0];
+        // in 32 bits (finish_plan keeps parts below 2^30): bounds and offsets of
+        // a stage formed in 64 bits cost the 28 columns of the C1 nmo-71 ladder
+        // 261 us instead of 231
+        const int kend = (int)(ke - kb);
         auto put_a = [&](int buf, int k, int m, i64 om, bool in, i64 ok) {
             stage_cp(&As[buf][k][m], in ? A + om + ok : A, in);
         };
@@ -155,42 +159,40 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
         };
         auto issue = [&](int s) {
             if (s < nst) {
-                const int buf = s % NST;
-                const i64 k0 = kb + (i64)s * BK;
-                const int left = (int)(ke - k0 < BK ? ke - k0 : BK);  // indices of this stage
+                const int buf = s % NST, k0 = s * BK;
                 if (afast) {  // a thread keeps its row (BM divides NT)
                     const int m = tid % BM;
                     const i64 om = offM[m];
 #pragma unroll
                     for (int i = 0; i < LA; i++) {
                         const int k = tid / BM + i * (NT / BM);
-                        put_a(buf, k, m, om, om >= 0 && k < left, lin ? (k0 + k) * ksa : offKA[buf][k]);
+                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksa : offKA[buf][k]);
                     }
                 } else {  // a thread keeps its contracted index
                     const int k = tid % BK;
-                    const i64 ok = lin ? (k0 + k) * ksa : offKA[buf][k];
+                    const i64 ok = lin ? (kb + k0 + k) * ksa : offKA[buf][k];
 #pragma unroll
                     for (int i = 0; i < LA; i++) {
                         const int m = tid / BK + i * (NT / BK);
                         const i64 om = offM[m];
-                        put_a(buf, k, m, om, om >= 0 && k < left, ok);
+                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, ok);
                     }
                 }
                 if (bfast) {
                     const int k = tid % BK;
-                    const i64 ok = lin ? (k0 + k) * ksb : offKB[buf][k];
+                    const i64 ok = lin ? (kb + k0 + k) * ksb : offKB[buf][k];
 #pragma unroll
                     for (int i = 0; i < LB; i++) {
                         const int n = tid / BK + i * (NT / BK);
                         const i64 on = offN[n];
-                        put_b(buf, k, n, on, on >= 0 && k < left, ok);
+                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, ok);
                     }
                 } else {
 #pragma unroll
                     for (int i = 0; i < LB; i++) {
                         const int e = tid + i * NT, n = e % BN, k = e / BN;
                         const i64 on = offN[n];
-                        put_b(buf, k, n, on, on >= 0 && k < left, lin ? (k0 + k) * ksb : offKB[buf][k]);
+                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksb : offKB[buf][k]);
                     }
                 }
             }

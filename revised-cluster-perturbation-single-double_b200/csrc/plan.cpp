@@ -91,7 +91,8 @@ namespace {
 // their partial sums' traffic; nothing beats the operand re-reads at 6 TB/s.
 // A part keeps at least two stages.  (The parts used to be as many as fill 592
 // tiles with 256 deep parts, whatever the wave: 70 tiles of the C1 nmo-71
-// ladder made 630, two full waves and a tenth of a third, 299 us, now 240; 36
+// ladder made 630, two full waves and a tenth of a third, 299 us, now 231 to
+// 234; 36
 // tiles of a C2v nmo-48 ring stayed 36, 37 us, now 24 with its reduction.)
 constexpr i64 TILE_CTAS[NTILE] = {2, 3, 2, 3, 2};
 constexpr double TILE_EFF[NTILE] = {0.66, 0.62, 0.64, 0.74, 0.45}, TILE_LONE[NTILE] = {0.42, 0.25, 0.42, 0.28, 0.17};
@@ -196,7 +197,8 @@ void finish_plan(ContractPlan *plan, std::vector<TaskDev> tasks, std::vector<Seg
     for (int ti = 0; ti < (int)tasks.size(); ti++) {
         const TaskDev &tk = tasks[ti];
         i64 mt = (tk.M + TBM - 1) / TBM, nt = (tk.N + TBN - 1) / TBN;
-        const i64 ns = std::min(split, std::max<i64>(1, tk.Ktot / minpart));
+        // (the kernel counts the indices of a part in 32 bits)
+        const i64 ns = std::max(std::min(split, std::max<i64>(1, tk.Ktot / minpart)), (tk.Ktot + (1 << 30) - 1) >> 30);
         for (i64 a = 0; a < mt; a++)
             for (i64 b = 0; b < nt; b++) {
                 if (ns > 1) {

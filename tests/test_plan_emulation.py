@@ -347,3 +347,19 @@ def test_plans_follow_the_product_table():
         got = emulate(tasks, segs, tiles, x[0], x[1], x[2], 1.0, tile)
         d = [dense.dpd_to_dense(y, sym, p, (1, 1), 1) for y, (_, p) in zip(x + [got], spec + spec[2:])]
         np.testing.assert_allclose(d[3], d[2] + np.einsum("aebf,eifj->aibj", d[0], d[1]), rtol=0, atol=1e-12)
+
+
+@pytest.mark.parametrize("m,n,e,f", [(1, 1, 40000, 60000), (20, 1, 40000, 30000), (17, 33, 70000, 70000)])
+def test_long_contracted_ranges_come_in_parts(m, n, e, f):
+    """The tile kernel counts the contracted indices of a tile in 32 bits: parts of at most 2^30."""
+    api.init(1, xor_dirprd(1))
+    pop = {c: np.array([k] + [0] * 7, np.int64) for c, k in zip("abefz", (m, n, e, f, 1))}
+    opts = []
+    for t in ("aezf", "ebfz", "abzz"):
+        opt = api.Opt()
+        api.check(api.lib().cpsd_opt_init(ctypes.byref(opt), *[api.arr8(pop[c]) for c in t], I64(1), I64(1), I64(1), None),
+                  "opt")
+        opts.append(opt)
+    tasks, _, tiles, _ = get_plan(opts[0], "ae.f", opts[1], "ebf.", opts[2], "ab..")
+    assert tasks[0].Ktot == e * f > 1 << 30
+    assert max(t.k_hi - t.k_lo for t in tiles) <= 1 << 30
