@@ -149,7 +149,9 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
         const i64 ksa = sg.kSA[0], ksb = sg.kSB[0];
         // in 32 bits (finish_plan keeps parts below 2^30): bounds and offsets of
         // a stage formed in 64 bits cost the 28 columns of the C1 nmo-71 ladder
-        // 261 us instead of 231
+        // (128x32) 261 us instead of 231, and a 128x64 ladder 568 instead of 553.
+        // The bound as what is left of the range suits the 64-row tiles (C2 nmo-74
+        // ladder 352 us, 369 as k0 + k < kend), not the 128-row ones (261, 558)
         const int kend = (int)(ke - kb);
         auto put_a = [&](int buf, int k, int m, i64 om, bool in, i64 ok) {
             stage_cp(&As[buf][k][m], in ? A + om + ok : A, in);
@@ -160,13 +162,14 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
         auto issue = [&](int s) {
             if (s < nst) {
                 const int buf = s % NST, k0 = s * BK;
+                const int at = BM == 64 ? 0 : k0, end = BM == 64 ? kend - k0 : kend;
                 if (afast) {  // a thread keeps its row (BM divides NT)
                     const int m = tid % BM;
                     const i64 om = offM[m];
 #pragma unroll
                     for (int i = 0; i < LA; i++) {
                         const int k = tid / BM + i * (NT / BM);
-                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksa : offKA[buf][k]);
+                        put_a(buf, k, m, om, om >= 0 && at + k < end, lin ? (kb + k0 + k) * ksa : offKA[buf][k]);
                     }
                 } else {  // a thread keeps its contracted index
                     const int k = tid % BK;
@@ -175,7 +178,7 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
                     for (int i = 0; i < LA; i++) {
                         const int m = tid / BK + i * (NT / BK);
                         const i64 om = offM[m];
-                        put_a(buf, k, m, om, om >= 0 && k0 + k < kend, ok);
+                        put_a(buf, k, m, om, om >= 0 && at + k < end, ok);
                     }
                 }
                 if (bfast) {
@@ -185,14 +188,14 @@ __global__ void __launch_bounds__(32 * WM * WN, WM * WN == 4 ? 3 : 2) k_contract
                     for (int i = 0; i < LB; i++) {
                         const int n = tid / BK + i * (NT / BK);
                         const i64 on = offN[n];
-                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, ok);
+                        put_b(buf, k, n, on, on >= 0 && at + k < end, ok);
                     }
                 } else {
 #pragma unroll
                     for (int i = 0; i < LB; i++) {
                         const int e = tid + i * NT, n = e % BN, k = e / BN;
                         const i64 on = offN[n];
-                        put_b(buf, k, n, on, on >= 0 && k0 + k < kend, lin ? (kb + k0 + k) * ksb : offKB[buf][k]);
+                        put_b(buf, k, n, on, on >= 0 && at + k < end, lin ? (kb + k0 + k) * ksb : offKB[buf][k]);
                     }
                 }
             }
