@@ -29,14 +29,6 @@ Context &ctx() {
     return c;
 }
 
-std::string sym_key() {
-    const i64 n = ctx().nirrep;
-    std::string s = "#";
-    for (i64 j = 1; j <= n; j++)
-        for (i64 i = 1; i <= n; i++) s += (char)('0' + dp(i, j));
-    return s;
-}
-
 // irpdso (src/libsrint/irpdso.f:1-52)
 i64 irpdso(i64 sym, const i64 *popp, const i64 *popq, i64 iop) {
     i64 n = 0;

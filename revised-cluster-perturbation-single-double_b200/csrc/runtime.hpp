@@ -31,6 +31,9 @@ struct Context {
     bool init = false;
     i64 nirrep = 1;
     i64 dirprd[8][8] = {};  // [i-1][j-1]
+    // irreps and their products, one character each (tables of eight irreps
+    // differ with the order of the irreps)
+    std::string sym_key;
     cudaStream_t stream = nullptr;
     int64_t launches = 0;
     double flops = 0;  // useful contraction flops issued (2 M N K per block)
@@ -50,9 +53,8 @@ struct Context {
 };
 Context &ctx();
 inline i64 dp(i64 a, i64 b) { return ctx().dirprd[a - 1][b - 1]; }
-// the symmetry as part of a plan's key: irreps and their products (tables of
-// eight irreps differ with the order of the irreps)
-std::string sym_key();
+// the symmetry as part of a plan's key
+inline const std::string &sym_key() { return ctx().sym_key; }
 inline cudaStream_t stream() { return ctx().stream; }
 inline void count_launch(int n = 1) { ctx().launches += n; }
 
