@@ -1226,10 +1226,9 @@ int cpsd_init(int64_t nirrep, const int64_t *dirprd) {
         for (int j = 1; j <= nirrep; j++)
             if (c.dirprd[i - 1][j - 1] < 1 || c.dirprd[i - 1][j - 1] > nirrep)
                 return set_error(CPSD_EARG, "cpsd_init: invalid direct-product table");
-    char key[64];
     for (int i = 0; i < nirrep; i++)
-        for (int j = 0; j < nirrep; j++) key[i * nirrep + j] = (char)('0' + c.dirprd[i][j]);
-    c.sym_key.assign(key, (size_t)(nirrep * nirrep));
+        for (int j = 0; j < nirrep; j++) c.sym_key[i * nirrep + j] = (char)('0' + c.dirprd[i][j]);
+    c.sym_key[nirrep * nirrep] = 0;
     c.init = true;
     return CPSD_OK;
 }

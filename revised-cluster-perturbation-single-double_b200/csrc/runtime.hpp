@@ -33,7 +33,9 @@ struct Context {
     i64 dirprd[8][8] = {};  // [i-1][j-1]
     // irreps and their products, one character each (tables of eight irreps
     // differ with the order of the irreps)
-    std::string sym_key;
+    // (plain characters: ctx() is called by the hundred for a launch, and a
+    // member with a constructor would put a check into each call)
+    char sym_key[72] = {};
     cudaStream_t stream = nullptr;
     int64_t launches = 0;
     double flops = 0;  // useful contraction flops issued (2 M N K per block)
@@ -54,7 +56,7 @@ struct Context {
 Context &ctx();
 inline i64 dp(i64 a, i64 b) { return ctx().dirprd[a - 1][b - 1]; }
 // the symmetry as part of a plan's key
-inline const std::string &sym_key() { return ctx().sym_key; }
+inline const char *sym_key() { return ctx().sym_key; }
 inline cudaStream_t stream() { return ctx().stream; }
 inline void count_launch(int n = 1) { ctx().launches += n; }
 
