@@ -198,10 +198,10 @@ __device__ void jacobi_place(double *S, int n, F a) {
 }
 
 // Cyclic Jacobi by the whole block on the symmetric n x n matrix that
-// jacobi_place put into S: w receives the eigenvalues, the columns of V (ld
-// GL) the eigenvectors; S2 and V2 are scratch of the same size.  The order of
-// the rotations is part of the result, as it decides the sign of every
-// eigenvector.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an element
+// jacobi_place put into S: w receives the eigenvalues; the eigenvector of w[k]
+// is column place[k] of the returned matrix (ld GL), which is V or V2.  S, S2,
+// V and V2 are of the same size.  The order of the rotations is part of the
+// result, as it decides the sign of every eigenvector.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an element
 // with a_pq^2 <= 1e-34 |a_pp a_qq| is negligible and set to zero.  The
 // n(n-1)/2 rotations of a sweep run as n-1 rounds of n/2 disjoint rotations
 // (round-robin pairing, n padded to even), each round one parallel update of
@@ -221,7 +221,7 @@ __device__ void jacobi_place(double *S, int n, F a) {
 // of the next round's pairing, in the other of two buffers: every address of
 // a thread is the same in all rounds.  (Indexing the pairs anew took 1250
 // cycles a round; roots, divisions and the index arithmetic 2000.)
-__device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n, double *w) {
+__device__ double *block_jacobi(double *S, double *V, double *S2, double *V2, int n, double *w, int *place) {
     __shared__ double cs[DAV_MAXD / 2], sn[DAV_MAXD / 2], tn[DAV_MAXD / 2];
     __shared__ int rotate;  // last round that saw an element above the threshold
     const int tid = threadIdx.x;
@@ -283,6 +283,8 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
     const bool dia = on_s && k0 == l0;
     double *A = S, *B = S2, *E = V, *F = V2;
     int r = 0;  // pairing of the round
+    // indices of this thread's rotation (the first half threads)
+    int pa = jacobi_at(2 * tid, m, 0), pb = tid;
     __syncthreads();
     for (int round = 1; round <= 50 * (m - 1); round++) {
         // does any element of the matrix still call for a rotation?
@@ -325,7 +327,7 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
             c = fma(0.5 * c, z, c);
             s = fma(0.5 * s, z, s);
             // equal diagonal elements: t = 1 from the lower to the higher index
-            if (d == 0.0 ? jacobi_at(2 * tid, m, r) > jacobi_at(2 * tid + 1, m, r) : (d > 0.0) != (b > 0.0)) s = -s;
+            if (d == 0.0 ? pa > pb : (d > 0.0) != (b > 0.0)) s = -s;
             cs[tid] = keep ? 1.0 : c;
             sn[tid] = keep ? 0.0 : s;
             tn[tid] = keep ? 0.0 : s * ru;  // s / c
@@ -366,23 +368,19 @@ __device__ void block_jacobi(double *S, double *V, double *S2, double *V2, int n
         E = F;
         F = x;
         r = r + 1 < m - 1 ? r + 1 : 0;
+        pa = tid == 0 ? pa : pa + 1 < m - 1 ? pa + 1 : 0;
+        pb = pb + 1 < m - 1 ? pb + 1 : 0;
         __syncthreads();
     }
-    // back from the places of the last pairing, two elements of V a thread
-    if (tid < m && jacobi_at(tid, m, r) < n) w[jacobi_at(tid, m, r)] = A[tid * (GL + 1)];
-    double v[2];
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-        const int e = tid + u * DT;
-        v[u] = E[e / DAV_MAXD * GL + e % DAV_MAXD];
+    if (tid < m) {
+        const int k = jacobi_at(tid, m, r);
+        if (k < n) {
+            w[k] = A[tid * (GL + 1)];
+            place[k] = tid;
+        }
     }
     __syncthreads();
-#pragma unroll
-    for (int u = 0; u < 2; u++) {
-        const int e = tid + u * DT, j = e % DAV_MAXD;
-        if (j < m) V[e / DAV_MAXD * GL + jacobi_at(j, m, r)] = v[u];
-    }
-    __syncthreads();
+    return E;
 }
 
 // ------------------------------------------------ general real eigenproblem
@@ -812,6 +810,7 @@ struct DavShared {
     double2 cf[DAV_MAXD][4];           // coefficients of eight outputs
     double vR[DAV_MAXD], vI[DAV_MAXD], ev[DAV_MAXD], rnorm[DAV_MAXD];
     int lw[DAV_MAXD], act[DAV_MAXD], cvd[DAV_MAXD];
+    int place[DAV_MAXD];  // column of an eigenvector
     int general, eig_fail, warn, nnew;
 };
 
@@ -946,8 +945,9 @@ __device__ void team_dots(DavShared &sm, int nc, const double *x, i64 ldx, int n
 __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int local) {
     extern __shared__ double dav_smem[];
     DavShared &sm = *reinterpret_cast<DavShared *>(dav_smem);
-    double *const S = sm.S, *const V = sm.V, *const X = sm.X, *const vR = sm.vR, *const vI = sm.vI;
-    int *const lw = sm.lw;
+    double *const S = sm.S, *const X = sm.X, *const vR = sm.vR, *const vI = sm.vI;
+    double *V = sm.V;  // eigenvector k in column place[k]; in sm.tot until the new vectors' sums go there
+    int *const lw = sm.lw, *const place = sm.place;
     DavState &s = *st;
     const int tid = threadIdx.x;
     const int D = s.D, n = s.dimA, nroot = s.nroot;
@@ -998,7 +998,7 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int
         __syncthreads();
         if (!general) {
             jacobi_place(S, dimIter, [&](int i, int j) { return 0.5 * (s.Abar[i + j * D] + s.Abar[j + i * D]); });
-            block_jacobi(S, V, X, sm.tot, dimIter, vR);
+            V = block_jacobi(S, V, X, sm.tot, dimIter, vR, place);
         } else {
             for (int e = tid; e < dimIter * dimIter; e += DT) {
                 const int i = e / dimIter, j = e % dimIter;
@@ -1006,6 +1006,7 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int
             }
             __syncthreads();
             if (tid < 32) {
+                place[tid] = tid;
                 const int sw = warp_geev(S, V, X, V, vR, vI, dimIter);
                 if (tid == 0) {
                     eig_fail = sw < 0;
@@ -1033,7 +1034,7 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int
         }
         return;
     }
-    // eigenvalues, their order and the chosen roots (vecR(i, k) = V[i][k])
+    // eigenvalues, their order and the chosen roots (vecR(i, k) = V[i][place[k]])
     // sort (mod_davidson.f90:620-640): position = number of smaller values;
     // equal values keep the order that the reference's exchanges leave
     if (tid < 32) {
@@ -1068,7 +1069,7 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int
         if (!s.lowest)
             for (int iroot = 0; iroot < nroot; iroot++) {
                 const int mine = tid < dimIter ? lw[tid] : 0;
-                double best = tid >= iroot && tid < dimIter ? fabs(V[iroot * GL + (mine - 1)]) : 0.0;
+                double best = tid >= iroot && tid < dimIter ? fabs(V[iroot * GL + place[mine - 1]]) : 0.0;
                 int at = best > 0.0 ? tid : iroot;
                 if (!(best > 0.0)) best = 0.0;
                 for (int o = 16; o > 0; o >>= 1) {
@@ -1094,7 +1095,7 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int
         const int nd = ndimIter;
         for (int e = tid; e < nd * dimIter; e += DT) {
             const int k = e % dimIter, i = e / dimIter;
-            S[i * GL + k] = V[k * GL + (lw[i] - 1)];
+            S[i * GL + k] = V[k * GL + place[lw[i] - 1]];
         }
         if (tid < nd) sm.act[tid] = tid;
         __syncthreads();
@@ -1155,7 +1156,7 @@ __global__ void __launch_bounds__(DT) k_dav_step(DavState *st, DavBuffers b, int
                 W1[ir * ld + k] = Bl[ir * ld + k];
             }
     } else {
-        combine(sm.cf, nc, dimIter, nroot, ABl, Bl, ld, [&](int i, int r) { return V[i * GL + (lw[r] - 1)]; },
+        combine(sm.cf, nc, dimIter, nroot, ABl, Bl, ld, [&](int i, int r) { return V[i * GL + place[lw[r] - 1]]; },
                 [&](int r, int k, double x, double y) {
                     W0[r * ld + k] = x;
                     W1[r * ld + k] = y;
@@ -1753,10 +1754,11 @@ __global__ void __launch_bounds__(32) k_geev_probe(const double *A, int n, doubl
 // the symmetric eigen-solve of the Davidson step on one given matrix
 __global__ void __launch_bounds__(DT) k_syev_probe(const double *A, int n, double *wr, double *V) {
     __shared__ double S[DAV_MAXD * GL], S2[DAV_MAXD * GL], U[DAV_MAXD * GL], U2[DAV_MAXD * GL], w[DAV_MAXD];
+    __shared__ int place[DAV_MAXD];
     jacobi_place(S, n, [&](int i, int j) { return A[i * n + j]; });
-    block_jacobi(S, U, S2, U2, n, w);
+    const double *const E = block_jacobi(S, U, S2, U2, n, w, place);
     if ((int)threadIdx.x < n) wr[threadIdx.x] = w[threadIdx.x];
-    for (int e = threadIdx.x; e < n * n; e += DT) V[e] = U[(e / n) * GL + e % n];
+    for (int e = threadIdx.x; e < n * n; e += DT) V[e] = E[(e / n) * GL + place[e % n]];
 }
 
 }  // namespace
