@@ -9,10 +9,10 @@
 // q stay in registers for the whole block, those over p are finished within
 // the strip.  Strips have a leading dimension of 4 mod 16 doubles, so that
 // both fragment shapes (8 p x 4 q and 8 q x 4 p) fall on different banks.
-// A warp only reads what it copied itself.  C2v nmo 151 (373 MB of list): 152 us a
-// launch; 204 us with the copies' addresses formed anew for every element (64
+// A warp only reads what it copied itself.  C2v nmo 151 (373 MB of list): 151 us a
+// call; 210 us with the copies' addresses formed anew for every element (64
 // instructions per 32 elements, issue-bound) and the strip's other loads not
-// ahead; expansion and row-dot contraction took 811 us.
+// ahead; expansion and row-dot contraction took 813 us.
 #include <algorithm>
 #include <map>
 #include <mutex>

@@ -91,8 +91,7 @@ namespace {
 // their partial sums' traffic; nothing beats the operand re-reads at 6 TB/s.
 // A part keeps at least two stages.  (The parts used to be as many as fill 592
 // tiles with 256 deep parts, whatever the wave: 70 tiles of the C1 nmo-71
-// ladder made 630, two full waves and a tenth of a third, 299 us, now 231 to
-// 234; 36
+// ladder made 630, two full waves and a tenth of a third, 299 us, now 231; 36
 // tiles of a C2v nmo-48 ring stayed 36, 37 us, now 24 with its reduction.)
 constexpr i64 TILE_CTAS[NTILE] = {2, 3, 2, 3, 2};
 constexpr double TILE_EFF[NTILE] = {0.66, 0.62, 0.64, 0.74, 0.45}, TILE_LONE[NTILE] = {0.42, 0.25, 0.42, 0.28, 0.17};

@@ -201,8 +201,9 @@ __device__ void jacobi_place(double *S, int n, F a) {
 // jacobi_place put into S: w receives the eigenvalues; the eigenvector of w[k]
 // is column place[k] of the returned matrix (ld GL), which is V or V2.  S, S2,
 // V and V2 are of the same size.  The order of the rotations is part of the
-// result, as it decides the sign of every eigenvector.  Classic threshold (Golub & Van Loan, Alg. 8.5.3): an element
-// with a_pq^2 <= 1e-34 |a_pp a_qq| is negligible and set to zero.  The
+// result, as it decides the sign of every eigenvector.  Classic threshold
+// (Golub & Van Loan, Alg. 8.5.3): an element with a_pq^2 <= 1e-34 |a_pp a_qq|
+// is negligible and set to zero.  The
 // n(n-1)/2 rotations of a sweep run as n-1 rounds of n/2 disjoint rotations
 // (round-robin pairing, n padded to even), each round one parallel update of
 // S and V.  The iteration ends at the first round whose matrix has no
@@ -283,7 +284,7 @@ __device__ double *block_jacobi(double *S, double *V, double *S2, double *V2, in
     const bool dia = on_s && k0 == l0;
     double *A = S, *B = S2, *E = V, *F = V2;
     int r = 0;  // pairing of the round
-    // indices of this thread's rotation (the first half threads)
+    // indices of this thread's rotation (threads below half)
     int pa = jacobi_at(2 * tid, m, 0), pb = tid;
     __syncthreads();
     for (int round = 1; round <= 50 * (m - 1); round++) {
@@ -1474,8 +1475,9 @@ __global__ void __launch_bounds__(DT) k_dav_final(DavState *st, DavBuffers b, co
 // LINPACK dgefa / dgesl (as MINV, src/libsrint/minv.f, calls them) by one
 // warp on a matrix in shared memory (n <= 32): lane i owns row i.  Pivot =
 // first row of largest magnitude, NaN counting as the largest (compared as it
-// is, it would leave the lanes with different rows and some with none); every element sees the same operations in
-// the same order as the sequential LINPACK loops.
+// is, it would leave the lanes with different rows and some with none); every
+// element sees the same operations in the same order as the sequential LINPACK
+// loops.
 __device__ void warp_dgefa(double *a, int lda, int n, int *ipvt) {
     const int i = threadIdx.x & 31;
     for (int k = 0; k < n - 1; k++) {
@@ -1558,7 +1560,7 @@ __device__ void block_reduce(const double (&v)[M], double (*red)[DT / 32], doubl
 // cluster.  Short R1 vectors are latency-bound (one CTA; up to three
 // exchanges a step), the (R1, R2) vectors of the grCPS(D) programs
 // bandwidth-bound: 2 x diis_dim stored vectors are read a step, by 16 SMs
-// (27 k elements: 165 us a step on one).
+// (26 k elements: 230 us a step on one SM, 33 on 16).
 //   1. R1 = pr / den and the sums of orthogonalR2L (R -= (<L|R> / ||L||) L:
 //      the reference divides by the norm, not its square) or <R1|nrmv>;
 //   2. that correction, the DIIS error vector and its overlaps;
